@@ -313,7 +313,11 @@ cudaError_t launch(spoc_handle *h, double *const s[3], const StageArgs &sa, cuda
   RhsBuffers b = rhs_buffers(h, s);
   if (q) b.q = q;
   b.sh_ready = sh_ready;
-  if (fast && h->precision == SPOC_FP64_FMA)
+  const bool fma = h->precision == SPOC_FP64_FMA;
+  if (fast && h->op.img_tile)
+    return (fma ? launch_rhs_tile_fma : launch_rhs_tile)(h->variant, h->op, h->mesh, b, sa, h->st,
+                                                         h->sms, &h->launches, ev);
+  if (fast && fma)
     return launch_rhs_fast_fma(h->variant, h->op, h->mesh, b, sa, h->st, h->sms, &h->launches,
                                ev);
   if (fast)
@@ -437,6 +441,15 @@ extern "C" int spoc_create(const spoc_tables *t, const spoc_mesh *m, int variant
       if (ce == cudaSuccess) ce = fast_build_images(h->op, img, imgq, h->st);
       h->op.img_ops = img;
       h->op.img_q = imgq;
+      if (ce == cudaSuccess && tile_pays(variant, nc, h->ng, h->ngf, h->ne, h->sms)) {
+        void *imgt = nullptr;
+        ce = h->alloc(reinterpret_cast<char **>(&imgt), tile_image_bytes(nc, h->ng, h->ngf));
+        if (ce == cudaSuccess) ce = tile_build_images(h->op, imgt, h->st);
+        if (ce == cudaSuccess) ce = h->alloc(&h->op.sched, kTileCounters);
+        if (ce == cudaSuccess)
+          ce = cudaMemsetAsync(h->op.sched, 0, sizeof(unsigned) * kTileCounters, h->st);
+        h->op.img_tile = imgt;
+      }
     }
     for (int c = 0; c < 3 && ce == cudaSuccess; ++c)
       ce = cudaMemsetAsync(h->U0[c], 0, sizeof(double) * n, h->st);
@@ -1355,7 +1368,9 @@ int adj_init(spoc_handle *h, AdjCtx *c) {
 // is one (bit-identical), else the generic one
 int base_q(spoc_handle *h, double *const s[3], double *q) {
   cudaError_t e = cudaErrorNotSupported;
-  if (h->path != SPOC_PATH_GENERIC && fast_available(h->nc, h->ng, h->ngf))
+  if (h->path != SPOC_PATH_GENERIC && h->op.img_tile)
+    e = launch_qphase_tile(h->variant, h->op, h->mesh, s[0], s[1], q, h->fv, h->st, h->sms);
+  else if (h->path != SPOC_PATH_GENERIC && fast_available(h->nc, h->ng, h->ngf))
     e = launch_qphase_fast(h->variant, h->op, h->mesh, s[0], s[1], q, h->st, h->sms);
   if (e == cudaErrorNotSupported)
     e = launch_qphase(h->variant, h->op, h->mesh, s[0], s[1], q, h->st, h->sms);

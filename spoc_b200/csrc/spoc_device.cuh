@@ -50,8 +50,12 @@ struct DevOps {
   // copy engine); null where the degree has no such kernels
   const void *img_ops;  // q-phase, tendency and linear kernels
   const void *img_q;    // quadrature-point kernel
+  const void *img_tile; // kernels with several elements per warp (null: not used)
+  unsigned *sched;      // their tile counters (kTileCounters, zero between launches)
   int *flag;            // the handle's error flags (bit 2: a wait limit ran out)
 };
+
+constexpr int kTileCounters = 6;
 
 // Mesh pointers with 0-based ids; -1 marks a wall in tseg.
 struct DevMesh {

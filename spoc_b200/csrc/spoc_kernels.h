@@ -211,6 +211,24 @@ cudaError_t launch_rhs_fast(int variant, const DevOps &op, const DevMesh &m, con
 cudaError_t launch_qphase_fast(int variant, const DevOps &op, const DevMesh &m, const double *su,
                                const double *sv, double *q, cudaStream_t st, int sms);
 
+// Kernels with several elements per warp (spoc_tile.cu) of the nonlinear
+// variants, tabulated sizes; identical results to launch_rhs_fast (the same
+// operations in the same order, fused multiply-adds in the _fma form).
+// Whether the mesh is large enough for them, the bytes of their operator
+// images, the kernel that writes them, one right-hand side or RK4 stage, and
+// the q-phase alone (fv: scratch, [nf][2][ngf] at least).
+bool tile_pays(int variant, int nc, int ng, int ngf, int ne, int sms);
+size_t tile_image_bytes(int nc, int ng, int ngf);
+cudaError_t tile_build_images(const DevOps &op, void *img, cudaStream_t st);
+cudaError_t launch_rhs_tile(int variant, const DevOps &op, const DevMesh &m, const RhsBuffers &b,
+                            const StageArgs &sa, cudaStream_t st, int sms, long long *launches,
+                            cudaEvent_t *ev = nullptr);
+cudaError_t launch_rhs_tile_fma(int variant, const DevOps &op, const DevMesh &m,
+                                const RhsBuffers &b, const StageArgs &sa, cudaStream_t st, int sms,
+                                long long *launches, cudaEvent_t *ev = nullptr);
+cudaError_t launch_qphase_tile(int variant, const DevOps &op, const DevMesh &m, const double *su,
+                               const double *sv, double *q, double *fv, cudaStream_t st, int sms);
+
 // Several RK4 steps of the linear variant in one cooperative launch of the
 // compile-time-sized kernel, bit-identical to one launch per stage; returns
 // cudaErrorNotSupported (nothing launched) when the degree is not tabulated
