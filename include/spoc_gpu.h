@@ -99,7 +99,9 @@ int spoc_create(const spoc_tables *tables, const spoc_mesh *mesh, int variant, i
 void spoc_destroy(spoc_handle *h);
 /* Kernel family (no reference counterpart; results are identical):
  * SPOC_PATH_AUTO picks the compile-time-sized kernels when (nc, ng, ngf) is
- * one of the tabulated combinations, else the generic runtime-sized ones. */
+ * one of the tabulated combinations, else the generic runtime-sized ones.
+ * SPOC_MIXED handles: SPOC_PATH_GENERIC keeps to one element per warp, the
+ * others choose several per warp on larger meshes. */
 #define SPOC_PATH_AUTO 0
 #define SPOC_PATH_GENERIC 1
 #define SPOC_PATH_TEMPLATED 2

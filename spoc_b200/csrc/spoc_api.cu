@@ -463,7 +463,7 @@ extern "C" int spoc_create(const spoc_tables *t, const spoc_mesh *m, int variant
   }
   if (!rc && precision == SPOC_MIXED) {
     std::string err;
-    rc = mixed_create(&h->mx, t, variant, h->ne, h->sms, &err);
+    rc = mixed_create(&h->mx, t, h->mesh, variant, h->sms, &err);
     if (rc) rc = fail(rc, err.c_str());
     if (!rc) {
       ce = mixed_set_state(h->mx, h->mesh, h->U0, h->st, &h->launches);
@@ -497,8 +497,8 @@ extern "C" int spoc_set_kernel_path(spoc_handle *h, int path) {
   if (!h || path < SPOC_PATH_AUTO || path > SPOC_PATH_TENSOR) return fail(SPOC_E_ARG, "bad argument");
   if (path == SPOC_PATH_TENSOR && (!h->mx || !mixed_set_tensor(h->mx, true)))
     return fail(SPOC_E_UNSUPPORTED, "tensor-core kernels: SPOC_MIXED, nonlinear variants, tabulated (nc, ng, ngf)");
-  if (h->mx && (path == SPOC_PATH_TEMPLATED || path == SPOC_PATH_GENERIC)) mixed_set_tensor(h->mx, false);
-  if (h->mx && path == SPOC_PATH_AUTO) mixed_default_path(h->mx);
+  if (h->mx && path == SPOC_PATH_GENERIC) mixed_one_element_path(h->mx);
+  if (h->mx && (path == SPOC_PATH_TEMPLATED || path == SPOC_PATH_AUTO)) mixed_default_path(h->mx);
   if (path == SPOC_PATH_TEMPLATED && !fast_available(h->nc, h->ng, h->ngf))
     return fail(SPOC_E_UNSUPPORTED, "no compile-time-sized kernels for this (nc, ng, ngf)");
   h->path = path;
@@ -1877,7 +1877,7 @@ extern "C" int spoc_set_adjoint_sweeps(spoc_handle *h, const spoc_tables *t, int
     return fail(SPOC_E_ARG, "no mixed-precision form at this degree");
   if (c->sweep_mx) return SPOC_OK;
   std::string err;
-  const int rc = mixed_create(&c->sweep_mx, t, h->variant, h->ne, h->sms, &err);
+  const int rc = mixed_create(&c->sweep_mx, t, h->mesh, h->variant, h->sms, &err);
   if (rc) {
     c->sweep_mx = nullptr;
     return fail(rc, err.c_str());

@@ -23,7 +23,9 @@
 // bases are FP64.
 //
 // Kernels (one warp per element, lanes over modes, quadrature points or the
-// 3*ngf face points; operators staged in shared memory per persistent block):
+// 3*ngf face points; operators staged in shared memory per persistent block;
+// larger meshes and ensembles run the same chains with several elements per
+// warp, spoc_mixed_tile.cu):
 //   kx_vol<VAR>  nonlinear variants, phases A, B and the volume parts of C, D
 //                of calvarnl_*.f (q, quadrature products, F and h volume
 //                terms), writing partial load vectors and the face traces of
@@ -33,7 +35,6 @@
 //   kx_lin       calvar_lin.f in one kernel.
 // Face values are the central averages of cal_flu, formed from traces that
 // each element writes for its own three sides (no face arrays).
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -96,9 +97,9 @@ __device__ __forceinline__ void sweep(int k0, const float *const (&x)[NX], F &&f
 
 // Trace record (mean-free traces, then the mean) of up to six fields held in
 // the warp's shared vectors x[f] (psi coefficients); written by lanes 0..TG.
-template <class Dm, int NF>
+template <class Dm, int NF, int FS>
 __device__ __forceinline__ void write_traces(const float *o, const float *const (&x)[NF], float *out,
-                                             size_t stride, int e) {
+                                             int e) {
   constexpr int N = Dm::N, TG = Dm::TG, TS = Dm::TS;
   const int lane = threadIdx.x & (Dm::LW - 1);
   if (lane > TG) return;
@@ -119,7 +120,7 @@ __device__ __forceinline__ void write_traces(const float *o, const float *const 
   }
   const size_t off = (size_t)e * TS + lane;
 #pragma unroll
-  for (int f = 0; f < NF; ++f) out[f * stride + off] = t[f];
+  for (int f = 0; f < NF; ++f) out[off * FS + f] = t[f];
 }
 
 // Orthogonal projection of the warp's vector x (shared, length N) onto the
@@ -218,15 +219,14 @@ __device__ void finish_element(const MxArgs &a, const float *o, float *w, int e,
   if (a.stage < 0) return;
   __syncwarp(lane_mask<Dm>());
   const float *const x[3] = {w, w + N, w + 2 * N};
-  write_traces<Dm, 3>(o, x, a.tr_out, (size_t)a.ne * Dm::TS, e);
+  write_traces<Dm, 3, kTr>(o, x, a.tr_out, e);
   __syncwarp(lane_mask<Dm>());
 }
 
 // ---------------------------------------------------------------------------
 // Nonlinear variants: volume kernel (calvarnl_fs.f:88-332 and the volume terms
 // of :341-544).
-// Body shared by kx_vol and the ensemble kernel: block blk of nblk working
-// on the elements of one member; the operators are already in sm.
+// The operators are already in sm.
 template <class Dm, int VAR>
 __device__ __forceinline__ void vol_body(const MxArgs &a, float *sm, int blk, int nblk) {
   constexpr int N = Dm::N, Q = Dm::Q, G = Dm::G, TG = Dm::TG, R = Dm::R;
@@ -236,7 +236,7 @@ __device__ __forceinline__ void vol_body(const MxArgs &a, float *sm, int blk, in
   float *su = w + Dm::S_U, *sv = w + Dm::S_V, *sh = w + Dm::S_H, *sq = w + Dm::S_Q;
   float *vec = w + Dm::S_VEC, *suh = w + Dm::S_UH, *svh = w + Dm::S_VH, *tmp = w + Dm::S_TMP;
   float *gl = w + Dm::S_GL, *qp = w + Dm::S_QP;
-  const size_t fn = (size_t)a.ne * N, tn = (size_t)a.ne * Dm::TS;
+  const size_t fn = (size_t)a.ne * N;
   const int stride = nblk * Dm::SLOTS;
   for (int e = blk * Dm::SLOTS + wib; e < a.ne; e += stride) {
     const double *vp = a.m.vect + 5 * (size_t)e;
@@ -252,8 +252,8 @@ __device__ __forceinline__ void vol_body(const MxArgs &a, float *sm, int blk, in
     if (lane < TG) {
       const int k = lane / G, j = lane - k * G;
       const FaceRef r = face_ref(a.m, e, k);
-      const float fu = face_value<G>(a.tr_in, r, e, lane, j);
-      const float fv = face_value<G>(a.tr_in + tn, r, e, lane, j);
+      const float fu = face_value<G, kTr>(a.tr_in, r, e, lane, j);
+      const float fv = face_value<G, kTr>(a.tr_in + 1, r, e, lane, j);
       const float s = r.sig * di * o[Dm::WIF + (r.sig > 0.f ? j : G - 1 - j)];
       gl[lane] = s * r.nx * fu;
       gl[TG + lane] = s * r.ny * fu;
@@ -539,7 +539,7 @@ __device__ __forceinline__ void vol_body(const MxArgs &a, float *sm, int blk, in
     // trace records of q and uh, vh for the face terms of phases C and D
     {
       const float *const x[6] = {sq, sq + N, sq + 2 * N, sq + 3 * N, suh, svh};
-      write_traces<Dm, 6>(o, x, a.trq, tn, e);
+      write_traces<Dm, 6, kTrq>(o, x, a.trq, e);
     }
     __syncwarp(lane_mask<Dm>());
   }
@@ -562,20 +562,20 @@ __device__ __forceinline__ void tend_body(const MxArgs &a, float *sm, int blk, i
   const int lane = threadIdx.x & (Dm::LW - 1), wib = threadIdx.x / Dm::LW;
   float *w = sm + Dm::NOPS + wib * Dm::WS;
   float *gl = w + Dm::S_GL, *tmp = w + Dm::S_TMP;
-  const size_t fn = (size_t)a.ne * N, tn = (size_t)a.ne * Dm::TS;
+  const size_t fn = (size_t)a.ne * N;
   const int stride = nblk * Dm::SLOTS;
   for (int e = blk * Dm::SLOTS + wib; e < a.ne; e += stride) {
     const float di = (float)a.m.vect[5 * (size_t)e + 4];
     if (lane < TG) {
       const int k = lane / G, j = lane - k * G;
       const FaceRef r = face_ref(a.m, e, k);
-      const float fqxx = face_value<G>(a.trq, r, e, lane, j);
-      const float fqxy = face_value<G>(a.trq + tn, r, e, lane, j);
-      const float fqyx = face_value<G>(a.trq + 2 * tn, r, e, lane, j);
-      const float fqyy = face_value<G>(a.trq + 3 * tn, r, e, lane, j);
-      const float fuh = face_value<G>(a.trq + 4 * tn, r, e, lane, j);
-      const float fvh = face_value<G>(a.trq + 5 * tn, r, e, lane, j);
-      const float fh = face_value<G>(a.tr_in + 2 * tn, r, e, lane, j);
+      const float fqxx = face_value<G, kTrq>(a.trq, r, e, lane, j);
+      const float fqxy = face_value<G, kTrq>(a.trq + 1, r, e, lane, j);
+      const float fqyx = face_value<G, kTrq>(a.trq + 2, r, e, lane, j);
+      const float fqyy = face_value<G, kTrq>(a.trq + 3, r, e, lane, j);
+      const float fuh = face_value<G, kTrq>(a.trq + 4, r, e, lane, j);
+      const float fvh = face_value<G, kTrq>(a.trq + 5, r, e, lane, j);
+      const float fh = face_value<G, kTr>(a.tr_in + 2, r, e, lane, j);
       const float Fxx = a.mu0 * fqxx - a.g0 * fh, Fxy = a.mu0 * fqxy;
       const float Fyx = a.mu0 * fqyx, Fyy = a.mu0 * fqyy - a.g0 * fh;
       const float s = r.sig * di * o[Dm::WIF + (r.sig > 0.f ? j : G - 1 - j)];
@@ -657,7 +657,7 @@ __global__ void __launch_bounds__(32 * kMxWarps, Dm::MINB_LIN) kx_lin(const MxAr
   float *w = sm + Dm::NOPS + wib * Dm::WS;
   float *su = w + Dm::S_U, *sv = w + Dm::S_V, *sh = w + Dm::S_H;
   float *gl = w + Dm::S_GL, *tmp = w + Dm::S_TMP;
-  const size_t fn = (size_t)a.ne * N, tn = (size_t)a.ne * Dm::TS;
+  const size_t fn = (size_t)a.ne * N;
   const int stride = gridDim.x * Dm::SLOTS;
   for (int e = blockIdx.x * Dm::SLOTS + wib; e < a.ne; e += stride) {
     const double *vp = a.m.vect + 5 * (size_t)e;
@@ -672,9 +672,9 @@ __global__ void __launch_bounds__(32 * kMxWarps, Dm::MINB_LIN) kx_lin(const MxAr
     if (lane < TG) {
       const int k = lane / G, j = lane - k * G;
       const FaceRef r = face_ref(a.m, e, k);
-      const float fu = face_value<G>(a.tr_in, r, e, lane, j);
-      const float fv = face_value<G>(a.tr_in + tn, r, e, lane, j);
-      const float fh = face_value<G>(a.tr_in + 2 * tn, r, e, lane, j);
+      const float fu = face_value<G, kTr>(a.tr_in, r, e, lane, j);
+      const float fv = face_value<G, kTr>(a.tr_in + 1, r, e, lane, j);
+      const float fh = face_value<G, kTr>(a.tr_in + 2, r, e, lane, j);
       const float s = r.sig * di * o[Dm::WIF + (r.sig > 0.f ? j : G - 1 - j)];
       const float fxx = -a.g0 * fh;
       gl[lane] = s * r.nx * fxx;
@@ -731,7 +731,7 @@ __global__ void __launch_bounds__(32 * kMxWarps, Dm::MINB) kx_prep(const MxArgs 
   __syncthreads();
   const int lane = threadIdx.x & (Dm::LW - 1), wib = threadIdx.x / Dm::LW;
   float *w = sm + Dm::NOPS + wib * Dm::WS;
-  const size_t fn = (size_t)a.ne * N, tn = (size_t)a.ne * Dm::TS;
+  const size_t fn = (size_t)a.ne * N;
   const int stride = gridDim.x * Dm::SLOTS;
   for (int e = blockIdx.x * Dm::SLOTS + wib; e < a.ne; e += stride) {
     for (int f = 0; f < 3; ++f)
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(32 * kMxWarps, Dm::MINB) kx_prep(const MxArgs 
       }
     __syncwarp(lane_mask<Dm>());
     const float *const x[3] = {w, w + N, w + 2 * N};
-    write_traces<Dm, 3>(o, x, a.tr_out, tn, e);
+    write_traces<Dm, 3, kTr>(o, x, a.tr_out, e);
     __syncwarp(lane_mask<Dm>());
   }
 }
@@ -790,7 +790,11 @@ struct MixedCtx {
   double *c64 = nullptr, *acc = nullptr, *k64 = nullptr, *cin = nullptr;
   float *y = nullptr, *tr[2]{}, *part = nullptr, *trq = nullptr;
   float *hbq = nullptr, *fcq = nullptr, *w0q = nullptr, *z0q = nullptr;
+  float *timg = nullptr;   // operator image of the kernels with several elements per warp
+  SideRef *refs = nullptr; // their side records
   float *tcimg = nullptr;  // operator image of the tensor-core volume kernel
+  bool tile_pays = false;  // the mesh is large enough for several elements per warp
+  bool tile = false;       // those kernels are used
   bool tc = false;         // nonlinear volume work on the tensor cores
   float psi0 = 0.f, wif[10]{};
   template <class T>
@@ -962,6 +966,14 @@ cudaError_t run_stage(MixedCtx *c, const MxArgs &a, cudaStream_t st, long long *
     if (launches) *launches += 1;
     return cudaGetLastError();
   }
+  if (c->tile && !c->tc) {
+    mark(0);
+    const cudaError_t te =
+        mixed_tile_rhs(c->variant, c->nc, c->Q, c->G, a, c->sms, st, ev ? ev[1] : nullptr);
+    mark(2);
+    if (te == cudaSuccess && launches) *launches += 2;
+    return te;
+  }
   cudaError_t tce = cudaSuccess;
   auto go = [&](MxKernel kv, MxKernel kt) {
     int gv = 0, gt = 0;
@@ -1018,6 +1030,8 @@ MxArgs base_args(MixedCtx *c, const DevMesh &m) {
   MxArgs a{};
   a.ne = c->ne;
   a.ops = c->ops;
+  a.timg = c->timg;
+  a.refs = c->refs;
   a.m = m;
   a.y = c->y;
   a.part = c->part;
@@ -1057,12 +1071,21 @@ bool mixed_set_tensor(MixedCtx *c, bool on) {
   return true;
 }
 
-void mixed_default_path(MixedCtx *c) { c->tc = false; }
+void mixed_default_path(MixedCtx *c) {
+  c->tc = false;
+  c->tile = c->tile_pays;
+}
+
+void mixed_one_element_path(MixedCtx *c) {
+  c->tc = false;
+  c->tile = false;
+}
 
 bool mixed_uses_tensor(const MixedCtx *c) { return c->tc; }
 
-int mixed_create(MixedCtx **out, const spoc_tables *t, int variant, int ne, int sms,
+int mixed_create(MixedCtx **out, const spoc_tables *t, const DevMesh &m, int variant, int sms,
                  std::string *err) {
+  const int ne = m.ne;
   *out = nullptr;
   if (!mixed_available(t->nc, t->ng, t->ngf)) {
     if (err) *err = "mixed precision is built for (nc, ng, ngf) = (3,12,4), (4,25,5), (5,27,6), (6,33,7), (7,42,9)";
@@ -1095,6 +1118,16 @@ int mixed_create(MixedCtx **out, const spoc_tables *t, int variant, int ne, int 
   if (ce == cudaSuccess && !tcimg.empty()) ce = c->alloc(&c->tcimg, tcimg.size());
   if (ce == cudaSuccess && !tcimg.empty())
     ce = cudaMemcpy(c->tcimg, tcimg.data(), sizeof(float) * tcimg.size(), cudaMemcpyHostToDevice);
+  if (variant != SPOC_LIN) {
+    const std::vector<float> timg = mixed_tile_image(t->nc, t->ng, t->ngf, p, t->wi, t->wif);
+    if (ce == cudaSuccess) ce = c->alloc(&c->timg, timg.size());
+    if (ce == cudaSuccess)
+      ce = cudaMemcpy(c->timg, timg.data(), sizeof(float) * timg.size(), cudaMemcpyHostToDevice);
+    c->tile = c->tile_pays = mixed_tile_pays(t->nc, t->ng, t->ngf, ne, sms);
+    if (ce == cudaSuccess) ce = c->alloc(&c->refs, 3 * (size_t)ne);
+    if (ce == cudaSuccess) ce = mixed_tile_refs(m, p.G, c->refs, nullptr);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(nullptr);
+  }
   // default kernel family: the FP32 pipes.  The tensor-core kernel is faster
   // at degree 7 but its three-term TF32 products are less accurate than FP32
   // multiply-adds (C3, 1000 steps: 1.0e-5 against 2.0e-6 relative eta
@@ -1109,10 +1142,10 @@ int mixed_create(MixedCtx **out, const spoc_tables *t, int variant, int ne, int 
   if (ce == cudaSuccess) ce = c->alloc(&c->k64, 3 * fn);
   if (ce == cudaSuccess) ce = c->alloc(&c->cin, 3 * fn);
   if (ce == cudaSuccess) ce = c->alloc(&c->y, 3 * fn);
-  if (ce == cudaSuccess) ce = c->alloc(&c->tr[0], 3 * tn);
-  if (ce == cudaSuccess) ce = c->alloc(&c->tr[1], 3 * tn);
+  if (ce == cudaSuccess) ce = c->alloc(&c->tr[0], kTr * tn);
+  if (ce == cudaSuccess) ce = c->alloc(&c->tr[1], kTr * tn);
   if (ce == cudaSuccess && variant != SPOC_LIN) ce = c->alloc(&c->part, 3 * fn);
-  if (ce == cudaSuccess && variant != SPOC_LIN) ce = c->alloc(&c->trq, 6 * tn);
+  if (ce == cudaSuccess && variant != SPOC_LIN) ce = c->alloc(&c->trq, kTrq * tn);
   if (ce == cudaSuccess) ce = c->alloc(&c->hbq, qn);
   if (ce == cudaSuccess) ce = c->alloc(&c->fcq, qn);
   if (ce == cudaSuccess) ce = c->alloc(&c->w0q, qn);
@@ -1228,67 +1261,7 @@ cudaError_t mixed_rhs(MixedCtx *c, const DevMesh &m, const double *const in[3],
 // operators once, runs the volume phase on the member's elements, waits for
 // the whole grid (the face terms of the tendency phase read neighbour trace
 // records), then runs the tendency phase.  All members are free-slip
-// (calvarnl_fs.f) and use the FP32-pipe kernels.
-
-struct EnsMember {
-  MxArgs a;        // stage, tr_in and tr_out are set per launch
-  float *tr[2];
-  int nc, first_block, nblocks;
-};
-
-namespace {
-
-template <class F>
-__device__ __forceinline__ void ens_dims(int nc, F &&f) {
-  switch (nc) {
-    case 3: f(MDims<3, 12, 4>{}); break;
-    case 4: f(MDims<4, 25, 5>{}); break;
-    case 5: f(MDims<5, 27, 6>{}); break;
-    default: f(MDims<6, 33, 7>{}); break;
-  }
-}
-
-constexpr int kEnsMinBlocks = 4;  // degrees 3-6: one row per lane, 64 registers
-
-// bt (null except when balancing): each block adds the SM cycles of its
-// volume phase (operator staging included) and of its tendency phase to
-// bt[2 b] and bt[2 b + 1].
-__global__ void __launch_bounds__(32 * kMxWarps, kEnsMinBlocks)
-    kx_ens_stage(const EnsMember *__restrict__ mem, const int *__restrict__ blk_member, int stage,
-                 int cur, unsigned long long *bt) {
-  extern __shared__ __align__(16) float sm[];
-  const EnsMember &em = mem[blk_member[blockIdx.x]];
-  MxArgs a = em.a;
-  a.stage = stage;
-  a.tr_in = em.tr[cur];
-  a.tr_out = em.tr[cur ^ 1];
-  const int lb = blockIdx.x - em.first_block, nb = em.nblocks;
-  const long long c0 = bt ? clock64() : 0;
-  ens_dims(em.nc, [&](auto d) { stage_mx_ops<decltype(d)>(sm, a.ops); });
-  __syncthreads();
-  ens_dims(em.nc, [&](auto d) { vol_body<decltype(d), SPOC_FS>(a, sm, lb, nb); });
-  if (bt) {
-    __syncthreads();
-    if (threadIdx.x == 0) atomicAdd(bt + 2 * blockIdx.x, (unsigned long long)(clock64() - c0));
-  }
-  cooperative_groups::this_grid().sync();
-  const long long c1 = bt ? clock64() : 0;
-  ens_dims(em.nc, [&](auto d) { tend_body<decltype(d), SPOC_FS>(a, sm, lb, nb); });
-  if (bt) {
-    __syncthreads();
-    if (threadIdx.x == 0) atomicAdd(bt + 2 * blockIdx.x + 1, (unsigned long long)(clock64() - c1));
-  }
-}
-
-size_t ens_smem() {
-  const size_t s[4] = {mx_smem<MDims<3, 12, 4>>(), mx_smem<MDims<4, 25, 5>>(),
-                       mx_smem<MDims<5, 27, 6>>(), mx_smem<MDims<6, 33, 7>>()};
-  size_t m = 0;
-  for (size_t v : s) m = v > m ? v : m;
-  return m;
-}
-
-}  // namespace
+// (calvarnl_fs.f); the kernel is in spoc_mixed_tile.cu.
 
 struct MixedEns {
   std::vector<MixedCtx *> mem;
@@ -1375,13 +1348,13 @@ int ens_layout(MixedEns *e) {
 }
 
 cudaError_t ens_launch_step(MixedEns *e, int cur0, unsigned long long *bt = nullptr) {
-  const size_t smem = ens_smem();
+  const EnsKernel k = mixed_tile_ens();
   for (int s = 0; s < 4; ++s) {
     int stage = s, cur = (cur0 + s) & 1;
     void *args[] = {(void *)&e->d_mem, (void *)&e->d_blk, (void *)&stage, (void *)&cur,
                     (void *)&bt};
-    cudaError_t ce = cudaLaunchCooperativeKernel((const void *)kx_ens_stage, dim3(e->nblk),
-                                                 dim3(32 * kMxWarps), args, smem, e->st);
+    cudaError_t ce = cudaLaunchCooperativeKernel(k.kernel, dim3(e->nblk), dim3(k.threads), args,
+                                                 k.smem, e->st);
     if (ce != cudaSuccess) return ce;
   }
   return cudaSuccess;
@@ -1411,12 +1384,12 @@ int mixed_ens_create(MixedEns **out, MixedCtx *const *ctx, const DevMesh *meshes
   e->flag.assign(flags, flags + n);
   e->dt.assign(n, 0.0);
   e->sms = sms;
-  const size_t smem = ens_smem();
-  cudaError_t ce = cudaFuncSetAttribute(kx_ens_stage, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem);
+  const EnsKernel k = mixed_tile_ens();
+  cudaError_t ce = cudaFuncSetAttribute(k.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)k.smem);
   int occ = 0;
   if (ce == cudaSuccess)
-    ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kx_ens_stage, 32 * kMxWarps, smem);
+    ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.kernel, k.threads, k.smem);
   if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking);
   if (ce != cudaSuccess || occ < 1) {
     if (err) *err = std::string("ensemble set-up: ") + cudaGetErrorString(ce);

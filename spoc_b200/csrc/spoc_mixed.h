@@ -24,8 +24,8 @@ struct MixedCtx;
 bool mixed_available(int nc, int ng, int ngf);
 
 // Builds the psi-basis operators from the COMMON-block tables and allocates
-// the device buffers for ne elements.
-int mixed_create(MixedCtx **out, const spoc_tables *t, int variant, int ne, int sms,
+// the device buffers for the mesh's elements.
+int mixed_create(MixedCtx **out, const spoc_tables *t, const DevMesh &m, int variant, int sms,
                  std::string *err);
 void mixed_destroy(MixedCtx *c);
 
@@ -57,8 +57,10 @@ int mixed_kernels_per_rhs(const MixedCtx *c);
 // Nonlinear volume kernel on the tensor cores (tcgen05) or on the FP32 pipes;
 // false if the tensor-core kernel is not available.
 bool mixed_set_tensor(MixedCtx *c, bool on);
-// back to the default family (FP32 pipes)
+// back to the default family (FP32 pipes), or to its one-element-per-warp
+// kernels whatever the mesh's size
 void mixed_default_path(MixedCtx *c);
+void mixed_one_element_path(MixedCtx *c);
 bool mixed_uses_tensor(const MixedCtx *c);
 
 // Ensemble of members (mixed precision, free-slip, degree 3-6) stepped

@@ -55,15 +55,30 @@ struct MDims {
   static_assert(N <= 64 && Q <= 64, "two rows per lane at most");
 };
 
+// One side of an element as the element sees it, laid out once per handle.
+struct __align__(16) SideRef {
+  int nb;     // neighbour, -1 for a wall
+  int at;     // trace index of the neighbour's point facing point 0 (points descend)
+  float sig;  // its * 0.5 (the tri_f factor)
+  float nx, ny;
+  int pad[3];
+};
+
+// Floats per point of the trace records: u, v, h and one unused; q (4), uh,
+// vh, the stage input's h (kernels with several elements per warp) and one unused.
+constexpr int kTr = 4, kTrq = 8;
+
 struct MxArgs {
   int ne;
   const float *ops;
+  const float *timg;    // operators of the kernels with several elements per warp
+  const SideRef *refs;  // [ne][3]
   DevMesh m;
-  const float *tr_in;  // [3][ne][TS] trace records of the stage input (u, v, h)
-  float *tr_out;       // [3][ne][TS] trace records of the next stage input
+  const float *tr_in;  // [ne][TS][kTr] trace records of the stage input (u, v, h)
+  float *tr_out;       // [ne][TS][kTr] trace records of the next stage input
   float *y;            // [3][ne][N] stage input (FP32); replaced by the next one
   float *part;         // [3][ne][N] partial load vectors (u, v, h)
-  float *trq;          // [6][ne][TS] trace records of qxx, qxy, qyx, qyy, uh, vh
+  float *trq;          // [ne][TS][kTrq] trace records of qxx, qxy, qyx, qyy, uh, vh (h)
   const float *hbq, *fcq, *w0q, *z0q;  // [ne][Q]; w0q / z0q null when zero
   float mu0, mb0, g0, hh0;
   int stage;           // 0..3 RK4 stage; -1: write the tendency to k64
@@ -117,13 +132,15 @@ __device__ __forceinline__ FaceRef face_ref(const DevMesh &m, int e, int k) {
 // point j of element e: own trace and the neighbour's trace at the mirrored
 // point (src/calflu.f:45-62); a wall face keeps the own trace
 // (src/calflu.f:35-39).
-template <int G>
+// tr: a record array at the field's offset, FS floats per point.
+template <int G, int FS>
 __device__ __forceinline__ float face_value(const float *tr, const FaceRef &r, int e, int l, int j) {
   constexpr int TG = 3 * G, TS = TG + 1;
-  const float own = tr[(size_t)e * TS + l];
+  const float own = tr[((size_t)e * TS + l) * FS];
   if (r.wall) return own;
-  const float *nb = tr + (size_t)r.nb * TS;
-  return 0.5f * (own + nb[r.s2 * G + (G - 1 - j)] + (nb[TG] - tr[(size_t)e * TS + TG]));
+  const float *nb = tr + (size_t)r.nb * TS * FS;
+  return 0.5f * (own + nb[(r.s2 * G + (G - 1 - j)) * FS] +
+                 (nb[TG * FS] - tr[((size_t)e * TS + TG) * FS]));
 }
 
 // RK4 bookkeeping of src/shwwnl.f:242-284 on one psi coefficient, FP64;
@@ -143,6 +160,14 @@ __device__ __forceinline__ double rk4_update(const MxArgs &a, size_t i, double d
   }
 }
 
+// A member of an ensemble as its kernel sees it: the kernel's arguments (stage,
+// tr_in and tr_out set per launch), the two trace buffers and its blocks.
+struct EnsMember {
+  MxArgs a;
+  float *tr[2];
+  int nc, first_block, nblocks;
+};
+
 }  // namespace mx
 
 // psi-basis operators built on the host in FP64 (spoc_mixed.cu).
@@ -159,5 +184,23 @@ cudaError_t mixed_tc_vol(int variant, int nc, int ng, int ngf, const mx::MxArgs 
 // The tendency kernel on the tensor cores (face lifts, wall projection, traces).
 cudaError_t mixed_tc_tend(int variant, int nc, int ng, int ngf, const mx::MxArgs &a, const float *img,
                          int sms, cudaStream_t st);
+
+// Kernels with several elements per warp (spoc_mixed_tile.cu): whether the mesh
+// is large enough for them, operator image, side records (3 ne of them) and
+// one right-hand side (mid: recorded between its two kernels, or null).
+bool mixed_tile_pays(int nc, int ng, int ngf, int ne, int sms);
+std::vector<float> mixed_tile_image(int nc, int ng, int ngf, const PsiOps &p, const double *wi,
+                                    const double *wif);
+// The ensemble kernel (EnsMember *, int *block member, int stage, int current
+// trace buffer, unsigned long long *block cycles), threads and shared memory.
+struct EnsKernel {
+  const void *kernel;
+  int threads;
+  size_t smem;
+};
+EnsKernel mixed_tile_ens();
+cudaError_t mixed_tile_refs(const DevMesh &m, int ngf, mx::SideRef *refs, cudaStream_t st);
+cudaError_t mixed_tile_rhs(int variant, int nc, int ng, int ngf, const mx::MxArgs &a, int sms,
+                           cudaStream_t st, cudaEvent_t mid);
 
 }  // namespace spoc

@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_vol(const MxArgs a, const fl
   const uint32_t tm = *slot;
   const uint32_t lrow = (uint32_t)((warp & 3) * 32) << 16;
   Pipe p{mbar, {0u, 0u}, {0u, 0u}, a.flag};
-  const size_t fn = (size_t)a.ne * N, tn = (size_t)a.ne * TS;
+  const size_t fn = (size_t)a.ne * N;
   // TMEM loads are issued in batches and completed with one wait
   auto ld = [&](int col, float (&v)[8]) { tc::tmem_ld8(tm + lrow + (uint32_t)col, v); };
   auto ldw = [&]() { tc::tmem_wait_ld(); };
@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_vol(const MxArgs a, const fl
     for (int f = 0; f < 2; ++f) {
       p.wait(0);
       p.wait(1);
-      const float *tr = a.tr_in + f * tn;
+      const float *tr = a.tr_in + f;
       // unrolled: the face of each point is known at compile time, so the
       // face references stay in registers
 #pragma unroll
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_vol(const MxArgs a, const fl
             if (valid && l < TG) {
               const int side = l / G, j = l - side * G;
               const FaceRef &r = fr[side];
-              const float fv = face_value<G>(tr, r, e, l, j);
+              const float fv = face_value<G, kTr>(tr, r, e, l, j);
               const float s = r.sig * di * a.wif[r.sig > 0.f ? j : G - 1 - j];
               x[jj] = s * r.nx * fv;
               z[jj] = s * r.ny * fv;
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_vol(const MxArgs a, const fl
       ldw();
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
-        float *rec = a.trq + f * tn + (size_t)(valid ? e : 0) * TS;
+        float *rec = a.trq + (size_t)(valid ? e : 0) * TS * kTrq + f;
         for (int c = 0; c < WT; c += 8)
           if (own(c)) {
             float v[8];
@@ -427,9 +427,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_vol(const MxArgs a, const fl
             ldw();
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              if (valid && c + j < TG) rec[c + j] = v[j];
+              if (valid && c + j < TG) rec[(c + j) * kTrq] = v[j];
           }
-        if (valid && half == 0) rec[TG] = a.psi0 * m[f][0];
+        if (valid && half == 0) rec[TG * kTrq] = a.psi0 * m[f][0];
       }
     }
 
@@ -649,7 +649,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_vol(const MxArgs a, const fl
       ldw();
 #pragma unroll
       for (int f = 0; f < 2; ++f) {
-        float *rec = a.trq + (4 + f) * tn + (size_t)(valid ? e : 0) * TS;
+        float *rec = a.trq + (size_t)(valid ? e : 0) * TS * kTrq + 4 + f;
         for (int c = 0; c < WT; c += 8)
           if (own(c)) {
             float v[8];
@@ -657,9 +657,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_vol(const MxArgs a, const fl
             ldw();
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              if (valid && c + j < TG) rec[c + j] = v[j];
+              if (valid && c + j < TG) rec[(c + j) * kTrq] = v[j];
           }
-        if (valid && half == 0) rec[TG] = a.psi0 * (f == 0 ? m0[0] : m1[0]);
+        if (valid && half == 0) rec[TG * kTrq] = a.psi0 * (f == 0 ? m0[0] : m1[0]);
       }
     }
     // the next tile waits on the A buffers before rewriting them; every TMEM
@@ -782,7 +782,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_tend(const MxArgs a, const f
   const uint32_t tm = *slot;
   const uint32_t lrow = (uint32_t)((warp & 3) * 32) << 16;
   Pipe3 p{mbar, {0u, 0u, 0u}, {0u, 0u, 0u}, a.flag};
-  const size_t fn = (size_t)a.ne * N, tn = (size_t)a.ne * TS;
+  const size_t fn = (size_t)a.ne * N;
   auto ld = [&](int col, float (&v)[8]) { tc::tmem_ld8(tm + lrow + (uint32_t)col, v); };
   auto ldw = [&]() { tc::tmem_wait_ld(); };
   auto abuf = [&](int b) { return sm + U::O_A + b * U::ABUF; };
@@ -834,13 +834,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_tend(const MxArgs a, const f
           if (valid && l < TG) {
             const int side = l / G, j = l - side * G;
             const FaceRef &r = fr[side];
-            const float fqxx = face_value<G>(a.trq, r, e, l, j);
-            const float fqxy = face_value<G>(a.trq + tn, r, e, l, j);
-            const float fqyx = face_value<G>(a.trq + 2 * tn, r, e, l, j);
-            const float fqyy = face_value<G>(a.trq + 3 * tn, r, e, l, j);
-            const float fuh = face_value<G>(a.trq + 4 * tn, r, e, l, j);
-            const float fvh = face_value<G>(a.trq + 5 * tn, r, e, l, j);
-            const float fh = face_value<G>(a.tr_in + 2 * tn, r, e, l, j);
+            const float fqxx = face_value<G, kTrq>(a.trq, r, e, l, j);
+            const float fqxy = face_value<G, kTrq>(a.trq + 1, r, e, l, j);
+            const float fqyx = face_value<G, kTrq>(a.trq + 2, r, e, l, j);
+            const float fqyy = face_value<G, kTrq>(a.trq + 3, r, e, l, j);
+            const float fuh = face_value<G, kTrq>(a.trq + 4, r, e, l, j);
+            const float fvh = face_value<G, kTrq>(a.trq + 5, r, e, l, j);
+            const float fh = face_value<G, kTr>(a.tr_in + 2, r, e, l, j);
             const float Fxx = a.mu0 * fqxx - a.g0 * fh, Fxy = a.mu0 * fqxy;
             const float Fyx = a.mu0 * fqyx, Fyy = a.mu0 * fqyy - a.g0 * fh;
             const float s = r.sig * di * a.wif[r.sig > 0.f ? j : G - 1 - j];
@@ -953,7 +953,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_tend(const MxArgs a, const f
         if (a.stage >= 0 && c == 0 && valid) {
           // the mean of each field: the constant mode's coefficient
 #pragma unroll
-          for (int f = 0; f < 3; ++f) a.tr_out[f * tn + (size_t)e * TS + TG] = a.psi0 * y[f][0];
+          for (int f = 0; f < 3; ++f) a.tr_out[((size_t)e * TS + TG) * kTr + f] = a.psi0 * y[f][0];
         }
       }
     if (bad) atomicOr(a.flag, 1);
@@ -970,7 +970,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_tend(const MxArgs a, const f
     p.wait_all();
 #pragma unroll
     for (int f = 0; f < 3; ++f) {
-      float *rec = a.tr_out + f * tn + (size_t)(valid ? e : 0) * TS;
+      float *rec = a.tr_out + (size_t)(valid ? e : 0) * TS * kTr + f;
       for (int c = 0; c < WT; c += 8)
         if (own(c)) {
           float v[8];
@@ -978,7 +978,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_tend(const MxArgs a, const f
           ldw();
 #pragma unroll
           for (int jj = 0; jj < 8; ++jj)
-            if (valid && c + jj < TG) rec[c + jj] = v[jj];
+            if (valid && c + jj < TG) rec[(c + jj) * kTr] = v[jj];
         }
     }
     // the trace columns are read before the next tile's lifts overwrite them

@@ -1,8 +1,10 @@
-"""The FP64 kernels with several elements per warp (spoc_tile.cu) against the
+"""Kernels with several elements per warp.  FP64 (spoc_tile.cu) against the
 CPU oracle, bit for bit: every tabulated degree and nonlinear variant on a mesh
 large enough for them whose element and face counts are not multiples of a
 tile, the smallest meshes that reach them (degree 4), and an odd element count
-at an odd mode count (fields aligned to 8 bytes only)."""
+at an odd mode count (fields aligned to 8 bytes only).  Mixed precision
+(spoc_mixed_tile.cu) against the one-element-per-warp kernels, which sum every
+chain in the same order: also bit for bit."""
 import numpy as np
 import pytest
 
@@ -76,3 +78,22 @@ def test_odd_element_count_bitwise(gpu_lib, nc, n):
     p = problem(nc, "fs", n, odd=True)
     assert p.mesh.ne % 2 == 1
     check(p)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("variant", ["fs", "ns", "inv"])
+@pytest.mark.parametrize("nc", sorted(RULES))
+def test_mixed_ragged_mesh_matches_one_element_kernels(gpu_lib, nc, variant):
+    p = problem(nc, variant, 41)
+    assert p.mesh.ne % 4 == 2
+    p.u, p.v, p.h = 0.1 * p.u, 0.1 * p.v, 0.1 * p.h
+    out = []
+    for path in ("auto", "generic"):
+        s = W.make_solver(p, "mixed")
+        s.set_kernel_path(path)
+        rhs = s.cal_var(p.u, p.v, p.h)
+        s.set_state(p.u, p.v, p.h)
+        s.rk4_steps(1.0e-3, 2)
+        out.append([*rhs, *s.get_state()])
+    for a, b in zip(*out):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
