@@ -69,7 +69,7 @@ struct spoc_handle {
   double *U0[3]{}, *SA[3]{}, *SB[3]{}, *ACC[3]{}, *TEND[3]{}, *SIN[3]{};
   double *hb = nullptr, *w0 = nullptr, *z0 = nullptr, *fc = nullptr;
   double *q = nullptr, *f = nullptr, *gx0 = nullptr, *gy0 = nullptr, *uh = nullptr, *vh = nullptr;
-  double *fv = nullptr;  // [nf][6][ngf] face values of the tendency kernel
+  double *fv = nullptr;  // [nf][6][ngf] face values of the tendency kernel ([nf][4][ngf]: linear)
   double *eterms = nullptr, *escal = nullptr;
   int *flag = nullptr;
   unsigned *gbar = nullptr;  // grid-barrier word of the multi-step linear kernel
@@ -443,7 +443,9 @@ extern "C" int spoc_create(const spoc_tables *t, const spoc_mesh *m, int variant
       h->op.img_q = imgq;
       if (ce == cudaSuccess && tile_pays(variant, nc, h->ng, h->ngf, h->ne, h->sms)) {
         void *imgt = nullptr;
-        ce = h->alloc(reinterpret_cast<char **>(&imgt), tile_image_bytes(nc, h->ng, h->ngf));
+        if (variant == SPOC_LIN) ce = h->alloc(&h->fv, 4 * (size_t)h->ngf * h->nf);
+        if (ce == cudaSuccess)
+          ce = h->alloc(reinterpret_cast<char **>(&imgt), tile_image_bytes(nc, h->ng, h->ngf));
         if (ce == cudaSuccess) ce = tile_build_images(h->op, imgt, h->st);
         if (ce == cudaSuccess) ce = h->alloc(&h->op.sched, kTileCounters);
         if (ce == cudaSuccess)

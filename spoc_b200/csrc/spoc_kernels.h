@@ -211,12 +211,13 @@ cudaError_t launch_rhs_fast(int variant, const DevOps &op, const DevMesh &m, con
 cudaError_t launch_qphase_fast(int variant, const DevOps &op, const DevMesh &m, const double *su,
                                const double *sv, double *q, cudaStream_t st, int sms);
 
-// Kernels with several elements per warp (spoc_tile.cu) of the nonlinear
-// variants, tabulated sizes; identical results to launch_rhs_fast (the same
+// Kernels with several elements per warp (spoc_tile.cu), tabulated sizes;
+// identical results to launch_rhs_fast (the same
 // operations in the same order, fused multiply-adds in the _fma form).
 // Whether the mesh is large enough for them, the bytes of their operator
 // images, the kernel that writes them, one right-hand side or RK4 stage, and
-// the q-phase alone (fv: scratch, [nf][2][ngf] at least).
+// the q-phase alone (fv: scratch, [nf][2][ngf] at least).  RhsBuffers::fv holds
+// [nf][6][ngf] values, [nf][4][ngf] for the linear variant.
 bool tile_pays(int variant, int nc, int ng, int ngf, int ne, int sms);
 size_t tile_image_bytes(int nc, int ng, int ngf);
 cudaError_t tile_build_images(const DevOps &op, void *img, cudaStream_t st);

@@ -1,5 +1,5 @@
-// Compile-time-sized FP64 kernels of the nonlinear right-hand sides, several
-// elements per warp.
+// Compile-time-sized FP64 kernels of the right-hand sides, several elements per
+// warp.
 //
 // Same arithmetic as spoc_kernels.cu (every sum in the reference order, every
 // product separately rounded, bit-identical results).  What bounds these
@@ -17,7 +17,8 @@
 //     and own their buffers, filled ahead with cp.async.
 // Measured against one element per warp (spoc_fast.cu) on 32768 triangles, us
 // per right-hand side: degree 3 217 -> 111, 4 358 -> 195, 5 493 -> 281,
-// 6 657 -> 419, 7 1390 -> 693.  The FP64 pipe is busy 55 to 63 % of the
+// 6 657 -> 419, 7 1390 -> 693; linear variant 98 -> 38, 132 -> 59, 177 -> 81,
+// 234 -> 119, 623 -> 177.  The FP64 pipe is busy 55 to 63 % of the
 // cycles; ptxas places a product's add right behind it, so a warp alone runs
 // at 44 % of the pipe's rate and three per scheduler (what the registers and
 // the shared memory hold) at about 90 % in the mat-vecs, less in the lifts
@@ -170,6 +171,10 @@ struct Degree {
   // 2048 (degree 3); 41 / 45 at 288 (degree 4); 61 / 60 at 1152, 63 / 70 at
   // 2048 (degree 5); 81 / 73 at 2048, 89 / 99 at 3200 (degree 6); 116 / 84 at
   // 1152, 121 / 132 at 2048 (degree 7)
+  // linear variant (one kernel there, two here): 24 / 21 at 2048 elements and
+  // 23 / 26 at 3200 (degree 4), 23 / 23 at 2048 (degree 5), 28 / 26 at 2048 and
+  // 32 / 36 at 3200 (degree 6), 37 / 52 at 2048 (degree 7)
+  static constexpr int MIN_PER_SM_LIN = 16;
   static constexpr int MIN_PER_SM = NC == 4 ? 0 : (NC == 6 ? 17 : (NC == 7 ? 13 : 10));
 };
 template <class P>
@@ -669,7 +674,8 @@ struct Tiles {
 // ---------------------------------------------------------------------------
 struct FaceArgs {
   const double *f[6];  // the fields, [ne][N] each
-  double *out;         // [nf][NF][G]
+  double *out;         // [nf][NF][G] (linear variant: [nf][4][G], the last unused)
+  double scale = 1.0;  // linear variant: factor of the first field's coefficients
 };
 
 template <class D, int FB>
@@ -681,6 +687,8 @@ template <class D, int NF, int FB, int W>
 __global__ void __launch_bounds__(32 * W) kt_faces(DevOps op, const OpsF<D> *img, DevMesh m,
                                                    FaceArgs fa) {
   constexpr int N = D::N, G = D::G, RF = D::RF, NB = NF / FB;
+  constexpr bool LIN = NF == 3;
+  constexpr int NR = LIN ? 4 : NF;  // fields of a record (16-byte aligned)
   static_assert(NB * FB == NF);
   extern __shared__ __align__(16) unsigned char smem[];
   OpsF<D> &S = *reinterpret_cast<OpsF<D> *>(smem);
@@ -776,8 +784,8 @@ __global__ void __launch_bounds__(32 * W) kt_faces(DevOps op, const OpsF<D> *img
 #pragma unroll
               for (int q = 0; q < FB; ++q) {
                 const double2 v = ld2(x + q * FE * D::SN + n);
-                c0[q] = v.x;
-                c1[q] = v.y;
+                c0[q] = LIN && q == 0 ? mul(fa.scale, v.x) : v.x;
+                c1[q] = LIN && q == 0 ? mul(fa.scale, v.y) : v.y;
               }
               mode(n, c0);
               mode(n + 1, c1);
@@ -787,7 +795,8 @@ __global__ void __launch_bounds__(32 * W) kt_faces(DevOps op, const OpsF<D> *img
             for (int n = 0; n < N; ++n) {
               double c0[FB];
 #pragma unroll
-              for (int q = 0; q < FB; ++q) c0[q] = x[q * FE * D::SN + n];
+              for (int q = 0; q < FB; ++q)
+                c0[q] = LIN && q == 0 ? mul(fa.scale, x[q * FE * D::SN + n]) : x[q * FE * D::SN + n];
               mode(n, c0);
             }
           }
@@ -801,7 +810,7 @@ __global__ void __launch_bounds__(32 * W) kt_faces(DevOps op, const OpsF<D> *img
           for (int r = 0; r < RF; ++r) {
             const int j = ls * RF + r;
             if (j < G)
-              fa.out[((size_t)f * NF + FB * b + q) * G + j] = wall ? acc[q][r] : mul(0.5, acc[q][r]);
+              fa.out[((size_t)f * NR + FB * b + q) * G + j] = wall ? acc[q][r] : mul(0.5, acc[q][r]);
           }
       }
     }
@@ -1282,6 +1291,162 @@ __global__ void __launch_bounds__(32 * W) kt_tendency(DevOps op, const OpsE<D> *
 }
 
 // ---------------------------------------------------------------------------
+// linear variant (calvar_lin.f:7-287) on the face values of -g0 h, u, v
+// ---------------------------------------------------------------------------
+template <class D>
+struct __align__(16) LWarp {
+  // stride of an element's three face records of four fields
+  static constexpr int SF = 12 * D::G + 2;
+  double own[3 * D::E * D::SN];  // h, u, v
+  double rec[D::E * SF];
+  double sm[D::E * D::SN];
+};
+
+template <class D, int W>
+__global__ void __launch_bounds__(32 * W) kt_linear(DevOps op, const OpsE<D> *img, DevMesh m, LinArgs a,
+                                                    const double *__restrict__ fv, StageArgs sa,
+                                                    unsigned *sched) {
+  constexpr int N = D::N, G = D::G, RN = D::RN, E = D::E, RG = D::RG, LR = Recs<D>::LR;
+  using LW = LWarp<D>;
+  extern __shared__ __align__(16) unsigned char smem[];
+  OpsE<D> &S = *reinterpret_cast<OpsE<D> *>(smem);
+  LW &w = reinterpret_cast<LW *>(smem + sizeof(OpsE<D>))[threadIdx.x >> 5];
+  const Lane l = lane_of<D>();
+  const int ntile = (m.ne + E - 1) / E;
+  Tiles<W> tiles(sched);
+  int tile = tiles.first();
+  auto issue = [&](int t, int face) {
+    const int part = lane_id() & 3, row = lane_id() >> 2;
+#pragma unroll
+    for (int i = 0; i < (3 * E + 7) / 8; ++i) {
+      const int r = row + 8 * i;
+      const double *f = r < E ? a.sh : (r < 2 * E ? a.su : a.sv);
+      if (r < 3 * E) copy_row<D>(w.own + r * D::SN, f + (size_t)min(t * E + r % E, m.ne - 1) * N, part);
+    }
+    const int k = lane_id() / LR, h = lane_id() % LR;
+    if (k < 3 * E) {
+      double *d = w.rec + (k / 3) * LW::SF + (k % 3) * 4 * G;
+#pragma unroll
+      for (int i = 0; i < 2 * G / LR; ++i) cp16(d + 2 * (h + LR * i), fv + (size_t)face * 4 * G + 2 * (h + LR * i));
+    }
+  };
+  if (tile < ntile) issue(tile, face_of_lane<D>(m, tile));
+  cp_commit();
+  __shared__ __align__(8) uint64_t ops_bar;
+  if (!bulk::stage_block(&S, img, sizeof(OpsE<D>), &ops_bar, op.flag)) {
+    cp_wait<0>();
+    return;
+  }
+  const double mg0 = -a.g0, hh0 = a.hh0;
+  for (int next; tile < ntile; tile = next) {
+    tiles.ask();
+    const int e = min(tile * E + l.e, m.ne - 1);
+    const bool live = tile * E + l.e < m.ne;
+    const Geo g = geo_of(m, e);
+    Sides sd;
+    sides_of(sd, m, e);
+    cp_wait<0>();
+    __syncwarp();
+    double t3[3][RN];
+    {
+      double x[3][RN], y[3][RN];  // agx, agy times fxx = fyy = -g0 h, u hh0, v hh0
+#pragma unroll
+      for (int f = 0; f < 3; ++f)
+#pragma unroll
+        for (int r = 0; r < RN; ++r) x[f][r] = y[f][r] = 0.0;
+      const double *c = w.own + l.e * D::SN;
+#pragma unroll 2
+      for (int j = 0; j < N; ++j) {
+        const double v[3] = {mul(mg0, c[j]), mul(c[E * D::SN + j], hh0), mul(c[2 * E * D::SN + j], hh0)};
+        const double *pa = S.ax + j * D::CW + 2 * l.s, *pb = S.ay + j * D::CW + 2 * l.s;
+#pragma unroll
+        for (int p = 0; p < (RN + 1) / 2; ++p) {
+          const double2 va = ld2(pa + p * 2 * RG), vb = ld2(pb + p * 2 * RG);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int r = 2 * p + h;
+            if (r >= RN) continue;
+#pragma unroll
+            for (int f = 0; f < 3; ++f) {
+              x[f][r] = macc(x[f][r], h ? va.y : va.x, v[f]);
+              y[f][r] = macc(y[f][r], h ? vb.y : vb.x, v[f]);
+            }
+          }
+        }
+      }
+      const double cby = mul(g.by, g.detai), cay = mul(g.ay, g.detai);
+      const double cbx = mul(g.bx, g.detai), cax = mul(g.ax, g.detai);
+#pragma unroll
+      for (int f = 0; f < 3; ++f)
+#pragma unroll
+        for (int r = 0; r < RN; ++r) t3[f][r] = 0.0;
+      // u, v (calvar_lin.f:143-166); the zero fields fxy, fyx contribute exact zeros
+      axpy(t3[0], x[0], -cby);
+      axpy(t3[0], y[0], cay);
+      axpy(t3[1], x[0], cbx);
+      axpy(t3[1], y[0], -cax);
+      // h (calvar_lin.f:256-270)
+      axpy(t3[2], x[1], cby);
+      axpy(t3[2], y[1], -cay);
+      axpy(t3[2], x[2], -cbx);
+      axpy(t3[2], y[2], cax);
+    }
+    next = tiles.next();
+    const int face = face_of_lane<D>(m, next < ntile ? next : tile);
+    // lifts: fbdxx, fbdyy of -g0 h; fbdx, fbdy of u, v, hh0 times
+    const double *fr = w.rec + l.e * LW::SF;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      double t[2][3][RN];
+#pragma unroll
+      for (int f = 0; f < 2; ++f)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+          for (int r = 0; r < RN; ++r) t[f][k][r] = 0.0;
+#pragma unroll 1
+      for (int jj = 0; jj < G; ++jj) {
+        const double wj = S.wif[jj];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const double *f = fr + k * 4 * G + jj;
+          const double fx = q == 0 ? mul(f[0], sd.nx[k]) : mul(mul(f[G], sd.nx[k]), hh0);
+          const double fy = q == 0 ? mul(f[0], sd.ny[k]) : mul(mul(f[2 * G], sd.ny[k]), hh0);
+          const double *pt =
+              S.pt + (sd.isg[k] < 0 ? OpsE<D>::PTS : 0) + (k * G + jj) * D::CW + 2 * l.s;
+#pragma unroll
+          for (int p = 0; p < (RN + 1) / 2; ++p) {
+            const double2 v = ld2(pt + p * 2 * RG);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const int r = 2 * p + h;
+              if (r >= RN) continue;
+              t[0][k][r] = macc(t[0][k][r], wj, mul(h ? v.y : v.x, fx));
+              t[1][k][r] = macc(t[1][k][r], wj, mul(h ? v.y : v.x, fy));
+            }
+          }
+        }
+      }
+      const double coeff = q == 0 ? g.detai : -g.detai;
+#pragma unroll
+      for (int f = 0; f < 2; ++f)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) axpy(t3[q == 0 ? f : 2], t[f][k], lift_sign(sd.isg[k], coeff));
+    }
+    __syncwarp();  // the buffer is free
+    if (next < ntile) issue(next, face);
+    cp_commit();
+    solve_vector<D, kINV, 3>(S.s, t3, g.wall, g.dnx, g.dny, w.sm, l);
+    StageRows<D> rows;
+    load_rows<D>(rows, sa, e, l);
+#pragma unroll
+    for (int f = 0; f < 3; ++f) stage_update<D>(sa, rows, f, e, live, t3[f], l);
+  }
+  cp_wait<0>();
+  tiles.done();
+}
+
+// ---------------------------------------------------------------------------
 // launch plumbing
 // ---------------------------------------------------------------------------
 // Warps of a block (one block per SM): as many as the shared memory holds
@@ -1377,6 +1542,30 @@ cudaError_t run_nl(const DevOps &op, const DevMesh &m, const RhsBuffers &b, cons
   return cudaSuccess;
 }
 
+template <class P>
+cudaError_t run_lin(const DevOps &op, const DevMesh &m, const RhsBuffers &b, const StageArgs &sa,
+                    cudaStream_t st, int sms, cudaEvent_t *ev, long long *launches) {
+  using D = typename P::DT;
+  const Images<P> *im = static_cast<const Images<P> *>(op.img_tile);
+  cudaError_t e = b.sh_ready ? cudaStreamWaitEvent(st, b.sh_ready, 0) : cudaSuccess;
+  if (ev && e == cudaSuccess) e = cudaEventRecord(ev[0], st);
+  const FaceArgs fa{{b.sh, b.su, b.sv}, b.fv, -b.g0};
+  if (e == cudaSuccess) e = run_faces<P, 3, 3>(op, im, m, fa, st, sms);
+  if (e != cudaSuccess) return e;
+  constexpr int W = warps(sizeof(OpsE<D>), sizeof(LWarp<D>), 12);
+  constexpr size_t sm = sizeof(OpsE<D>) + W * sizeof(LWarp<D>);
+  const auto k = kt_linear<D, W>;
+  int grid = 0;
+  e = tile_grid(k, W, sm, sms, (m.ne + D::E - 1) / D::E, &grid);
+  if (e != cudaSuccess) return e;
+  const LinArgs la{b.su, b.sv, b.sh, b.g0, b.hh0};
+  k<<<grid, 32 * W, sm, st>>>(op, &im->t, m, la, b.fv, sa, op.sched + 4);
+  e = cudaGetLastError();
+  if (ev && e == cudaSuccess) e = cudaEventRecord(ev[1], st);
+  *launches += 2;
+  return e;
+}
+
 template <class F>
 bool with_dims(int nc, int ng, int ngf, F &&f) {
   if (nc == 3 && ng == 12 && ngf == 4) return f(Degree<3, 12, 4>{}), true;
@@ -1396,8 +1585,10 @@ bool with_dims(int nc, int ng, int ngf, F &&f) {
 
 bool tile_pays(int variant, int nc, int ng, int ngf, int ne, int sms) {
   bool pays = false;
-  if (variant != kLIN)
-    with_dims(nc, ng, ngf, [&](auto d) { pays = ne >= decltype(d)::MIN_PER_SM * sms; });
+  with_dims(nc, ng, ngf, [&](auto d) {
+    using P = decltype(d);
+    pays = ne >= (variant == kLIN ? P::MIN_PER_SM_LIN : P::MIN_PER_SM) * sms;
+  });
   return pays;
 }
 
@@ -1443,7 +1634,7 @@ cudaError_t LAUNCH_TILE(int variant, const DevOps &op, const DevMesh &m, const R
       case kFS: e = run_nl<P, kFS>(op, m, b, sa, st, sms, ev, launches); break;
       case kNS: e = run_nl<P, kNS>(op, m, b, sa, st, sms, ev, launches); break;
       case kINV: e = run_nl<P, kINV>(op, m, b, sa, st, sms, ev, launches); break;
-      default: break;
+      default: e = run_lin<P>(op, m, b, sa, st, sms, ev, launches); break;
     }
   });
   return e;

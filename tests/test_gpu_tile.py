@@ -1,5 +1,5 @@
 """Kernels with several elements per warp.  FP64 (spoc_tile.cu) against the
-CPU oracle, bit for bit: every tabulated degree and nonlinear variant on a mesh
+CPU oracle, bit for bit: every tabulated degree and variant on a mesh
 large enough for them whose element and face counts are not multiples of a
 tile, the smallest meshes that reach them (degree 4), and an odd element count
 at an odd mode count (fields aligned to 8 bytes only).  Mixed precision
@@ -57,10 +57,11 @@ def check(p):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("variant", ["fs", "ns", "inv"])
+@pytest.mark.parametrize("variant", ["lin", "fs", "ns", "inv"])
 @pytest.mark.parametrize("nc", sorted(RULES))
 def test_ragged_mesh_bitwise(gpu_lib, nc, variant):
-    p = problem(nc, variant, 37)
+    # linear runs of up to 20 elements per SM take the multi-step kernel
+    p = problem(nc, variant, 41 if variant == "lin" else 37)
     assert p.mesh.ne % 4 and p.mesh.nf % 16
     check(p)
 
