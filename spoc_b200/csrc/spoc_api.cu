@@ -87,18 +87,42 @@ struct spoc_handle {
   double graph_key[6] = {};
   long long graph_launches = 0;
 
+  // Device memory of the handle comes in chunks that grow with it (2 MiB, then
+  // as much as is held already, up to 64 MiB at a time): a handle makes some
+  // fifty allocations of a few KiB to a few MiB, and a cudaMalloc and cudaFree
+  // pair costs 0.1 to 1 ms each.
+  char *chunk = nullptr;
+  size_t chunk_left = 0, held = 0;
   template <class T>
   cudaError_t alloc(T **p, size_t n) {
-    cudaError_t e = cudaMalloc((void **)p, sizeof(T) * (n ? n : 1));
-    if (e == cudaSuccess) allocs.push_back((void *)*p);
-    return e;
+    const size_t bytes = (sizeof(T) * (n ? n : 1) + 511) / 512 * 512;
+    if (bytes > chunk_left) {
+      const size_t grow = std::min<size_t>(std::max<size_t>(held, 2u << 20), 64u << 20);
+      const size_t size = std::max(bytes, grow);
+      void *q = nullptr;
+      const cudaError_t e = cudaMalloc(&q, size);
+      if (e != cudaSuccess) return e;
+      allocs.push_back(q);
+      held += size;
+      if (size - bytes >= chunk_left) {  // the fuller of the two chunks is left behind
+        chunk = static_cast<char *>(q) + bytes;
+        chunk_left = size - bytes;
+      }
+      *p = static_cast<T *>(q);
+      return cudaSuccess;
+    }
+    *p = reinterpret_cast<T *>(chunk);
+    chunk += bytes;
+    chunk_left -= bytes;
+    return cudaSuccess;
   }
   template <class T>
   cudaError_t upload(const T **p, const std::vector<T> &v) {
     T *d = nullptr;
-    cudaError_t e = dev_upload(&d, v);
-    if (d) allocs.push_back((void *)d);
+    cudaError_t e = alloc(&d, v.size());
     *p = d;
+    if (e == cudaSuccess && !v.empty())
+      e = cudaMemcpy(d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice);
     return e;
   }
   ~spoc_handle() {
@@ -850,6 +874,27 @@ int graph_steps_fp64(spoc_handle *h, double dt, int nsteps) {
   return SPOC_OK;
 }
 
+// The steps of spoc_rk4_steps_host: the first waits for h's upload, the last
+// stores to the caller's arrays; those between are replayed from the step
+// graph (20 launches a step otherwise, which small and middling meshes wait
+// for: 57 us a step by launches against 37 from the graph at degree 5 on 4050
+// triangles).  Short runs that would have to capture it first go without.
+int run_steps_host(spoc_handle *h, double dt, int nsteps, double *const *host, int ld,
+                   cudaEvent_t sh_ready) {
+  constexpr int kGraphFrom = 8;
+  bool one_launch = false;
+  if (h->variant == SPOC_LIN) {
+    const StageArgs probe{};
+    one_launch = lin_steps(h, probe, 0, nullptr, nullptr) == cudaSuccess;
+  }
+  if (one_launch || nsteps < (h->step_graph ? 3 : kGraphFrom))
+    return enqueue_steps_fp64(h, dt, nsteps, nullptr, host, ld, sh_ready);
+  int rc = enqueue_steps_fp64(h, dt, 1, nullptr, nullptr, 0, sh_ready);
+  if (!rc) rc = graph_steps_fp64(h, dt, nsteps - 2);
+  if (!rc) rc = enqueue_steps_fp64(h, dt, 1, nullptr, host, ld);
+  return rc;
+}
+
 int enqueue_steps(spoc_handle *h, double dt, int nsteps) {
   if (h->mx) {
     CK(mixed_steps(h->mx, h->mesh, dt, nsteps, h->flag, h->st, &h->launches), "mixed RK4 steps");
@@ -901,7 +946,7 @@ extern "C" int spoc_rk4_steps_host(spoc_handle *h, int ld, double *u, double *v,
     CK(cudaEventRecord(h->side_ev, h->side), "record");
     double *dh[3] = {nullptr, nullptr, nullptr};
     direct = mapped_host(u, &dh[0]) && mapped_host(v, &dh[1]) && mapped_host(hh, &dh[2]);
-    rc = enqueue_steps_fp64(h, dt, nsteps, nullptr, direct ? dh : nullptr, ld, h->side_ev);
+    rc = run_steps_host(h, dt, nsteps, direct ? dh : nullptr, ld, h->side_ev);
     if (rc) cudaStreamWaitEvent(h->st, h->side_ev, 0);  // leave no copy behind the stream
   }
   if (rc) return rc;

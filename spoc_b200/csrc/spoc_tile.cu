@@ -189,13 +189,12 @@ template <class F>
 __device__ void fill_factor(F &o, const double *rows, const double *cols, const double *dia, int ld) {
   using P = Pack<F::RG>;
   constexpr int N = F::N;
-  for (int k = 0; k < N; ++k) {
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
-      if (P::first(i) >= P::first(k))
-        o.f[P::fwd(k, even(F::RN)) + P::row(i) - P::first(k) * 2 * F::RG] = rows[k * ld + i];
-      if (P::first(i) <= P::first(k)) o.b[P::bwd(k) + P::row(i)] = cols[k * ld + i];
-    }
-    if (threadIdx.x == 0) o.dia[k] = dia[k];
+  for (int t = threadIdx.x; t < N * N; t += blockDim.x) {
+    const int k = t / N, i = t - k * N;
+    if (P::first(i) >= P::first(k))
+      o.f[P::fwd(k, even(F::RN)) + P::row(i) - P::first(k) * 2 * F::RG] = rows[k * ld + i];
+    if (P::first(i) <= P::first(k)) o.b[P::bwd(k) + P::row(i)] = cols[k * ld + i];
+    if (t < N) o.dia[t] = dia[t];
   }
 }
 template <class D>
