@@ -87,15 +87,21 @@ struct spoc_handle {
   double graph_key[6] = {};
   long long graph_launches = 0;
 
-  // Device memory of the handle comes in chunks that grow with it (2 MiB, then
-  // as much as is held already, up to 64 MiB at a time): a handle makes some
-  // fifty allocations of a few KiB to a few MiB, and a cudaMalloc and cudaFree
-  // pair costs 0.1 to 1 ms each.
+  // Allocations of 256 KiB and more come from chunks that grow with the handle
+  // (2 MiB, then as much as is held already, up to 64 MiB at a time): a handle
+  // makes some thirty of them, and each cudaMalloc and cudaFree pair maps and
+  // unmaps memory for 0.1 to 1 ms.  (Smaller ones cost microseconds: the
+  // runtime serves them from its own slabs.)
   char *chunk = nullptr;
   size_t chunk_left = 0, held = 0;
   template <class T>
   cudaError_t alloc(T **p, size_t n) {
     const size_t bytes = (sizeof(T) * (n ? n : 1) + 511) / 512 * 512;
+    if (bytes < (256u << 10)) {
+      const cudaError_t e = cudaMalloc((void **)p, bytes);
+      if (e == cudaSuccess) allocs.push_back((void *)*p);
+      return e;
+    }
     if (bytes > chunk_left) {
       const size_t grow = std::min<size_t>(std::max<size_t>(held, 2u << 20), 64u << 20);
       const size_t size = std::max(bytes, grow);
@@ -362,6 +368,10 @@ int check_flag(spoc_handle *h) {
   return SPOC_OK;
 }
 
+int build_lin_order(spoc_handle *h);
+cudaError_t small_steps(spoc_handle *h, const StageArgs &sa, int nsteps, double *const *host,
+                        cudaEvent_t sh_ready);
+
 int run_rhs_tend(spoc_handle *h, double *const s[3]) {
   if (h->mx) {
     CK(mixed_rhs(h->mx, h->mesh, s, h->TEND, h->flag, h->st, &h->launches), "mixed cal_var");
@@ -371,6 +381,12 @@ int run_rhs_tend(spoc_handle *h, double *const s[3]) {
   sa.stage = -1;
   for (int c = 0; c < 3; ++c) sa.tend[c] = h->TEND[c];
   sa.flag = h->flag;
+  if (h->variant != SPOC_LIN) {
+    for (int c = 0; c < 3; ++c) sa.base[c] = s[c];
+    const cudaError_t e = small_steps(h, sa, 1, nullptr, nullptr);
+    if (e == cudaSuccess) return SPOC_OK;
+    if (e != cudaErrorNotSupported) return fail(SPOC_E_CUDA, "launch cal_var", e);
+  }
   CK(launch(h, s, sa, nullptr), "launch cal_var");
   return SPOC_OK;
 }
@@ -745,41 +761,58 @@ int build_lin_order(spoc_handle *h) {
   return SPOC_OK;
 }
 
-// The linear variant on the compile-time-sized path runs all the steps in one
-// cooperative launch when the mesh fits one pass of the resident warps
-// (cudaErrorNotSupported: it does not, nothing was launched; nsteps 0 only
-// asks whether it applies).
-cudaError_t lin_steps(spoc_handle *h, const StageArgs &sa, int nsteps, double *const *host,
-                      cudaEvent_t sh_ready) {
-  if (h->variant != SPOC_LIN || h->path == SPOC_PATH_GENERIC ||
-      !fast_available(h->nc, h->ng, h->ngf))
+// The compile-time-sized path runs all the steps of a small mesh in one
+// cooperative launch (cudaErrorNotSupported: it does not apply, nothing was
+// launched; nsteps 0 only asks).
+cudaError_t small_steps(spoc_handle *h, const StageArgs &sa, int nsteps, double *const *host,
+                        cudaEvent_t sh_ready) {
+  if (h->path == SPOC_PATH_GENERIC || !fast_available(h->nc, h->ng, h->ngf))
     return cudaErrorNotSupported;
   // a cooperative launch is not captured into a caller's graph
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   cudaError_t e = cudaStreamIsCapturing(h->st, &cap);
   if (e != cudaSuccess) return e;
   if (cap != cudaStreamCaptureStatusNone) return cudaErrorNotSupported;
-  LinSteps ls{};
-  ls.sa = sa;
-  for (int c = 0; c < 3; ++c) {
-    ls.bufa[c] = h->SA[c];
-    ls.bufb[c] = h->SB[c];
-    ls.host[c] = host ? host[c] : nullptr;
+  const bool fma = h->precision == SPOC_FP64_FMA;
+  auto wait = [&] { return sh_ready ? cudaStreamWaitEvent(h->st, sh_ready, 0) : cudaSuccess; };
+  if (h->variant == SPOC_LIN) {
+    LinSteps ls{};
+    ls.sa = sa;
+    for (int c = 0; c < 3; ++c) {
+      ls.bufa[c] = h->SA[c];
+      ls.bufb[c] = h->SB[c];
+      ls.host[c] = host ? host[c] : nullptr;
+    }
+    ls.g0 = h->g0;
+    ls.hh0 = h->hh0;
+    ls.nsteps = nsteps;
+    ls.count = h->gbar;
+    if (!h->lin_order && build_lin_order(h)) return cudaErrorUnknown;
+    ls.order = h->lin_order;
+    ls.norder = h->lin_norder;
+    if ((e = wait()) != cudaSuccess) return e;
+    return (fma ? lin_steps_fast_fma : lin_steps_fast)(h->op, h->mesh, ls, h->st, h->sms, &h->launches);
   }
-  ls.g0 = h->g0;
-  ls.hh0 = h->hh0;
-  ls.nsteps = nsteps;
-  ls.count = h->gbar;
-  if (!h->lin_order && build_lin_order(h)) return cudaErrorUnknown;
-  ls.order = h->lin_order;
-  ls.norder = h->lin_norder;
-  if (sh_ready) {
-    e = cudaStreamWaitEvent(h->st, sh_ready, 0);
+  NlSteps ns{};
+  ns.sa = sa;
+  for (int c = 0; c < 3; ++c) {
+    ns.bufa[c] = h->SA[c];
+    ns.bufb[c] = h->SB[c];
+    ns.host[c] = host ? host[c] : nullptr;
+  }
+  ns.nl = NlArgs{nullptr, nullptr, nullptr, h->hb, h->w0, h->z0, h->fc, nullptr, h->gx0, h->gy0,
+                 h->uh, h->vh, h->f, h->mu0, h->mb0, h->g0};
+  ns.nsteps = nsteps;
+  ns.count = h->gbar;
+  auto go = fma ? nl_steps_fast_fma : nl_steps_fast;
+  if (nsteps > 0) {  // does it apply?
+    NlSteps probe = ns;
+    probe.nsteps = 0;
+    e = go(h->variant, h->op, h->mesh, probe, h->st, h->sms, &h->launches);
+    if (e == cudaSuccess) e = wait();
     if (e != cudaSuccess) return e;
   }
-  return h->precision == SPOC_FP64_FMA
-             ? lin_steps_fast_fma(h->op, h->mesh, ls, h->st, h->sms, &h->launches)
-             : lin_steps_fast(h->op, h->mesh, ls, h->st, h->sms, &h->launches);
+  return go(h->variant, h->op, h->mesh, ns, h->st, h->sms, &h->launches);
 }
 
 int enqueue_steps_fp64(spoc_handle *h, double dt, int nsteps, double *const *base = nullptr,
@@ -796,9 +829,9 @@ int enqueue_steps_fp64(spoc_handle *h, double dt, int nsteps, double *const *bas
   }
   sa.host_ld = host_ld;
   if (nsteps > 0) {
-    const cudaError_t le = lin_steps(h, sa, nsteps, host, sh_ready);
+    const cudaError_t le = small_steps(h, sa, nsteps, host, sh_ready);
     if (le == cudaSuccess) return SPOC_OK;
-    if (le != cudaErrorNotSupported) return fail(SPOC_E_CUDA, "multi-step linear launch", le);
+    if (le != cudaErrorNotSupported) return fail(SPOC_E_CUDA, "multi-step launch", le);
   }
   for (int it = 0; it < nsteps; ++it) {
     for (int s = 0; s < 4; ++s) {
@@ -827,10 +860,10 @@ int enqueue_steps_fp64(spoc_handle *h, double dt, int nsteps, double *const *bas
 // capture; the graph is captured from the next one.
 int graph_steps_fp64(spoc_handle *h, double dt, int nsteps) {
   if (nsteps <= 0) return SPOC_OK;
-  if (h->variant == SPOC_LIN) {
-    // the multi-step linear kernel needs no graph (nsteps 0: does it apply?)
+  {
+    // the multi-step kernels need no graph (nsteps 0: do they apply?)
     const StageArgs probe{};
-    if (lin_steps(h, probe, 0, nullptr, nullptr) == cudaSuccess)
+    if (small_steps(h, probe, 0, nullptr, nullptr) == cudaSuccess)
       return enqueue_steps_fp64(h, dt, nsteps);
   }
   // a caller capturing the handle's stream itself gets plain launches
@@ -882,11 +915,8 @@ int graph_steps_fp64(spoc_handle *h, double dt, int nsteps) {
 int run_steps_host(spoc_handle *h, double dt, int nsteps, double *const *host, int ld,
                    cudaEvent_t sh_ready) {
   constexpr int kGraphFrom = 8;
-  bool one_launch = false;
-  if (h->variant == SPOC_LIN) {
-    const StageArgs probe{};
-    one_launch = lin_steps(h, probe, 0, nullptr, nullptr) == cudaSuccess;
-  }
+  const StageArgs probe{};
+  const bool one_launch = small_steps(h, probe, 0, nullptr, nullptr) == cudaSuccess;
   if (one_launch || nsteps < (h->step_graph ? 3 : kGraphFrom))
     return enqueue_steps_fp64(h, dt, nsteps, nullptr, host, ld, sh_ready);
   int rc = enqueue_steps_fp64(h, dt, 1, nullptr, nullptr, 0, sh_ready);

@@ -193,7 +193,7 @@ __device__ __forceinline__ unsigned tile_mask() {
 
 // own field: lanes load v[e*N + i] into sm[i]
 template <class Dm>
-__device__ __forceinline__ void load_vec(double *sm, const double *__restrict__ g, int e) {
+__device__ __forceinline__ void load_vec(double *sm, const double *g, int e) {
   const int l = tile_lane<Dm::LW>();
 #pragma unroll
   for (int r = 0; r < Dm::R; ++r) {
@@ -203,7 +203,7 @@ __device__ __forceinline__ void load_vec(double *sm, const double *__restrict__ 
 }
 
 template <class Dm>
-__device__ __forceinline__ void load_reg(double (&x)[Dm::R], const double *__restrict__ g, int e) {
+__device__ __forceinline__ void load_reg(double (&x)[Dm::R], const double *g, int e) {
   const int l = tile_lane<Dm::LW>();
 #pragma unroll
   for (int r = 0; r < Dm::R; ++r) {
@@ -1278,6 +1278,100 @@ __device__ __forceinline__ void stage_update_sm(const StageArgs &sa, int fld, in
   }
 }
 
+// One element of the tendency phase: own / nb hold the element's and its
+// neighbours' six fields (FACES: nb holds the face records of kf_faces,
+// [side][field][point]); load_gxy(gx, gy) gives its gx0, gy0; after_volume()
+// runs once own, nb and those rows are free; gx, gy, hb receive the
+// tendencies of u, v, h.
+template <class Dm, int VAR, bool FACES = false, class LoadGxy, class AfterVolume>
+__device__ __forceinline__ void tend_elem(const SOps<Dm> &S, const DevMesh &m, int e, const Sides &sd,
+                                          const double *own, const double *nb, double *fb, double *sm,
+                                          LoadGxy load_gxy, AfterVolume after_volume,
+                                          double (&gx)[Dm::R], double (&gy)[Dm::R],
+                                          double (&hb)[Dm::R]) {
+  constexpr int N = Dm::N, R = Dm::R, G = Dm::G;
+  const Geo g = geo(m, e);
+  int isg[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) isg[k] = __ldg(m.its + 3 * e + k);
+  if constexpr (FACES) {
+    const int l = lane_id();
+    if (l < 3 * G) {
+      const int k = l / G, j = l - k * G;
+#pragma unroll
+      for (int f = 0; f < 6; ++f) fb[f * 32 + l] = nb[(k * 6 + f) * G + j];
+    }
+  } else {
+    face_values<Dm, 6>(S.pf, m, sd, own, nb, fb);
+  }
+  __syncwarp();
+  // each lane scales the values it computed (fbd * norm(1|2, face))
+#pragma unroll
+  for (int f = 0; f < 6; ++f) scale_face<Dm>(m, sd, fb + 32 * f, fb + 32 * f, f & 1);
+  double ax[6][R], bx[6][R];
+  matvec2<Dm, 6>(S.agx, S.agy, own, N, ax, bx);
+  load_gxy(gx, gy);
+  const double cby = mul(g.by, g.detai), cay = mul(g.ay, g.detai);
+  const double cbx = mul(g.bx, g.detai), cax = mul(g.ax, g.detai);
+  axpy<R>(gx, ax[0], -cby);
+  axpy<R>(gx, bx[0], cay);
+  axpy<R>(gx, ax[1], cbx);
+  axpy<R>(gx, bx[1], -cax);
+  axpy<R>(gy, ax[2], -cby);
+  axpy<R>(gy, bx[2], cay);
+  axpy<R>(gy, ax[3], cbx);
+  axpy<R>(gy, bx[3], -cax);
+#pragma unroll
+  for (int r = 0; r < R; ++r) hb[r] = 0.0;
+  axpy<R>(hb, ax[4], cby);
+  axpy<R>(hb, bx[4], -cay);
+  axpy<R>(hb, ax[5], -cbx);
+  axpy<R>(hb, bx[5], cax);
+  __syncwarp();  // own / nb and the gx0, gy0 rows are free from here on
+  after_volume();
+  double t[6][3][R];
+  lift_sums<Dm, 6>(S, isg, fb, t);
+  apply_lift<R>(gx, t[0], isg, g.detai);
+  apply_lift<R>(gx, t[1], isg, g.detai);
+  apply_lift<R>(gy, t[2], isg, g.detai);
+  apply_lift<R>(gy, t[3], isg, g.detai);
+  apply_lift<R>(hb, t[4], isg, -g.detai);
+  apply_lift<R>(hb, t[5], isg, -g.detai);
+  if (__ldg(m.bdl + e)) {
+    if (VAR == kNS) {
+      double bu[2][R], hs[1][R];
+      reduc<Dm>(S, gx, bu[0], sm);
+      reduc<Dm>(S, gy, bu[1], sm);
+      solve_red_b<Dm, SOps<Dm>, 2>(S, bu);
+      copy<R>(hs[0], hb);
+      solve_full_b<Dm, SOps<Dm>, 1>(S, hs);
+      copy<R>(hb, hs[0]);
+      reduc_inv<Dm>(S, bu[0], gx, sm);
+      reduc_inv<Dm>(S, bu[1], gy, sm);
+    } else {
+      const double dnx = __ldg(m.normt + 2 * e), dny = __ldg(m.normt + 2 * e + 1);
+      double gn[R], full2[2][R], bu[1][R];
+      rot<R>(gn, full2[0], gx, gy, dnx, dny);
+      copy<R>(full2[1], hb);
+      reduc<Dm>(S, gn, bu[0], sm);
+      solve_red_b<Dm, SOps<Dm>, 1>(S, bu);
+      solve_full_b<Dm, SOps<Dm>, 2>(S, full2);
+      reduc_inv<Dm>(S, bu[0], gn, sm);
+      rot<R>(gx, gy, gn, full2[0], dnx, dny);
+      copy<R>(hb, full2[1]);
+    }
+  } else {
+    double s3[3][R];
+    copy<R>(s3[0], gx);
+    copy<R>(s3[1], gy);
+    copy<R>(s3[2], hb);
+    solve_full_b<Dm, SOps<Dm>, 3>(S, s3);
+    copy<R>(gx, s3[0]);
+    copy<R>(gy, s3[1]);
+    copy<R>(hb, s3[2]);
+  }
+}
+
 template <class Dm, int VAR, bool FACES = false>
 __device__ __forceinline__ void tend_body(DevOps op, DevMesh m, TendArgs a, StageArgs sa) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -1320,10 +1414,6 @@ __device__ __forceinline__ void tend_body(DevOps op, DevMesh m, TendArgs a, Stag
     const Sides sd = PF ? sd_next : sides_of(m, e);
     const int en = e + warp_count();
     if (PF && en < m.ne) sd_next = sides_of(m, en);
-    const Geo g = geo(m, e);
-    int isg[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) isg[k] = __ldg(m.its + 3 * e + k);
     if constexpr (PF) {
       const bool ok = rows.wait(op.flag);
       cp_async_wait_all();
@@ -1334,92 +1424,25 @@ __device__ __forceinline__ void tend_body(DevOps op, DevMesh m, TendArgs a, Stag
       stage_neighbours<Dm, 6>(sd, W.nb, [&](int f, int t, int i) { return src[f][(size_t)t * N + i]; });
     }
     __syncwarp();
-    if constexpr (FACES) {
-      const int l = lane_id();
-      if (l < 3 * G) {
-        const int k = l / G, j = l - k * G;
-#pragma unroll
-        for (int f = 0; f < 6; ++f) W.fb[f * 32 + l] = W.fvs[(k * 6 + f) * G + j];
-      }
-    } else {
-      face_values<Dm, 6>(S.pf, m, sd, W.own, W.nb, W.fb);
-    }
-    __syncwarp();
-    // each lane scales the values it computed (fbd * norm(1|2, face))
-#pragma unroll
-    for (int f = 0; f < 6; ++f) scale_face<Dm>(m, sd, W.fb + 32 * f, W.fb + 32 * f, f & 1);
-    double ax[6][R], bx[6][R];
-    matvec2<Dm, 6>(S.agx, S.agy, W.own, N, ax, bx);
     double gx[R], gy[R], hb[R];
-    if constexpr (PF) {
-      gx[0] = lane_id() < N ? W.aux[lane_id()] : 0.0;
-      gy[0] = lane_id() < N ? W.aux[N + lane_id()] : 0.0;
-    } else {
-      load_reg<Dm>(gx, a.gx0, e);
-      load_reg<Dm>(gy, a.gy0, e);
-    }
-    const double cby = mul(g.by, g.detai), cay = mul(g.ay, g.detai);
-    const double cbx = mul(g.bx, g.detai), cax = mul(g.ax, g.detai);
-    axpy<R>(gx, ax[0], -cby);
-    axpy<R>(gx, bx[0], cay);
-    axpy<R>(gx, ax[1], cbx);
-    axpy<R>(gx, bx[1], -cax);
-    axpy<R>(gy, ax[2], -cby);
-    axpy<R>(gy, bx[2], cay);
-    axpy<R>(gy, ax[3], cbx);
-    axpy<R>(gy, bx[3], -cax);
-#pragma unroll
-    for (int r = 0; r < R; ++r) hb[r] = 0.0;
-    axpy<R>(hb, ax[4], cby);
-    axpy<R>(hb, bx[4], -cay);
-    axpy<R>(hb, ax[5], -cbx);
-    axpy<R>(hb, bx[5], cax);
-    __syncwarp();  // W.own / W.nb and the gx0, gy0 rows are free from here on
-    if (PF && en < m.ne) {
-      issue(rows, src, en, sd_next);
-      prefetch_gxy<Dm>(a, en, W.aux);
-    }
-    double t[6][3][R];
-    lift_sums<Dm, 6>(S, isg, W.fb, t);
-    apply_lift<R>(gx, t[0], isg, g.detai);
-    apply_lift<R>(gx, t[1], isg, g.detai);
-    apply_lift<R>(gy, t[2], isg, g.detai);
-    apply_lift<R>(gy, t[3], isg, g.detai);
-    apply_lift<R>(hb, t[4], isg, -g.detai);
-    apply_lift<R>(hb, t[5], isg, -g.detai);
-    if (__ldg(m.bdl + e)) {
-      if (VAR == kNS) {
-        double bu[2][R], hs[1][R];
-        reduc<Dm>(S, gx, bu[0], W.sm);
-        reduc<Dm>(S, gy, bu[1], W.sm);
-        solve_red_b<Dm, SOps<Dm>, 2>(S, bu);
-        copy<R>(hs[0], hb);
-        solve_full_b<Dm, SOps<Dm>, 1>(S, hs);
-        copy<R>(hb, hs[0]);
-        reduc_inv<Dm>(S, bu[0], gx, W.sm);
-        reduc_inv<Dm>(S, bu[1], gy, W.sm);
-      } else {
-        const double dnx = __ldg(m.normt + 2 * e), dny = __ldg(m.normt + 2 * e + 1);
-        double gn[R], full2[2][R], bu[1][R];
-        rot<R>(gn, full2[0], gx, gy, dnx, dny);
-        copy<R>(full2[1], hb);
-        reduc<Dm>(S, gn, bu[0], W.sm);
-        solve_red_b<Dm, SOps<Dm>, 1>(S, bu);
-        solve_full_b<Dm, SOps<Dm>, 2>(S, full2);
-        reduc_inv<Dm>(S, bu[0], gn, W.sm);
-        rot<R>(gx, gy, gn, full2[0], dnx, dny);
-        copy<R>(hb, full2[1]);
-      }
-    } else {
-      double s3[3][R];
-      copy<R>(s3[0], gx);
-      copy<R>(s3[1], gy);
-      copy<R>(s3[2], hb);
-      solve_full_b<Dm, SOps<Dm>, 3>(S, s3);
-      copy<R>(gx, s3[0]);
-      copy<R>(gy, s3[1]);
-      copy<R>(hb, s3[2]);
-    }
+    tend_elem<Dm, VAR, FACES>(
+        S, m, e, sd, W.own, FACES ? W.fvs : W.nb, W.fb, W.sm,
+        [&](double(&x)[R], double(&y)[R]) {
+          if constexpr (PF) {
+            x[0] = lane_id() < N ? W.aux[lane_id()] : 0.0;
+            y[0] = lane_id() < N ? W.aux[N + lane_id()] : 0.0;
+          } else {
+            load_reg<Dm>(x, a.gx0, e);
+            load_reg<Dm>(y, a.gy0, e);
+          }
+        },
+        [&] {
+          if (PF && en < m.ne) {
+            issue(rows, src, en, sd_next);
+            prefetch_gxy<Dm>(a, en, W.aux);
+          }
+        },
+        gx, gy, hb);
     if constexpr (PF) {
       stage_update_sm<Dm>(sa, 0, e, gx[0], W.aux);
       stage_update_sm<Dm>(sa, 1, e, gy[0], W.aux);
@@ -1770,6 +1793,148 @@ __global__ void __launch_bounds__(32 * MAXW) kf_lin_steps(DevOps op, DevMesh m, 
 }
 
 // ---------------------------------------------------------------------------
+// Small meshes, nonlinear variants: several RK4 steps (or one right-hand side)
+// in one cooperative launch, one element per warp for the whole launch.  Five
+// launches a stage cost more than the work of a few hundred elements, and
+// every launch stages its operators again; here they are staged once, the
+// element's state stays in registers, its quadrature-point phase follows its
+// q-phase in the same warp, and the grid meets twice a stage: before the
+// tendencies (neighbours' F, uh, vh) and after the stage update (neighbours'
+// stage input).  The element functions are those of the per-stage kernels.
+// ---------------------------------------------------------------------------
+template <class Dm>
+struct __align__(16) NWarp {
+  double rows[4 * Dm::N];  // hb, w0, z0, fc for the whole launch
+  union {
+    struct {
+      double own[2 * Dm::N], nb[3 * nb_stride<Dm, 2>()], fr[2 * 32], fb[4 * 32];
+    } q;
+    struct {
+      double rows[11 * Dm::N], vin[9 * Dm::N], wp[8 * Dm::Q], tail[9 * BWarp<Dm>::T];
+    } b;
+    struct {
+      double own[6 * Dm::N], nb[3 * nb_stride<Dm, 6>()], fb[6 * 32];
+    } t;
+  };
+  double sm[64];
+};
+
+// MAXW: the most warps per block the instance is built for
+template <class Dm, int VAR, int MAXW>
+__global__ void __launch_bounds__(32 * MAXW, 1) kf_nl_steps(DevOps op, DevMesh m, NlSteps ns) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  SOps<Dm> &S = *reinterpret_cast<SOps<Dm> *>(smem);
+  SOpsQ<Dm> &SQ = *reinterpret_cast<SOpsQ<Dm> *>(smem + sizeof(SOps<Dm>));
+  NWarp<Dm> &W = reinterpret_cast<NWarp<Dm> *>(smem + sizeof(SOps<Dm>) + sizeof(SOpsQ<Dm>))[warp_in_block()];
+  constexpr int N = Dm::N, R = Dm::R;
+  static_assert(R == 1, "one row per lane");
+  __shared__ __align__(8) uint64_t bar1, bar2;
+  const bool s1 = bulk::stage_block(&S, op.img_ops, sizeof(SOps<Dm>), &bar1, op.flag);
+  const bool s2 = bulk::stage_block(&SQ, op.img_q, sizeof(SOpsQ<Dm>), &bar2, op.flag);
+  const int l = lane_id(), e = blockIdx.x + gridDim.x * warp_in_block();
+  const bool active = s1 && s2 && e < m.ne;
+  const size_t fs = (size_t)m.ne * N;
+  const StageArgs &sa = ns.sa;
+  Sides sd{};
+  double u0[3][R], acc[3][R], x[3][R];  // u0, du1 + 2 du2 + 2 du3, stage input
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int r = 0; r < R; ++r) u0[c][r] = acc[c][r] = x[c][r] = 0.0;
+  if (active) {
+    sd = sides_of(m, e);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      load_reg<Dm>(u0[c], sa.base[c], e);
+      copy<R>(x[c], u0[c]);
+    }
+    const double *const fields[4] = {ns.nl.hb, ns.nl.w0, ns.nl.z0, ns.nl.fc};
+#pragma unroll
+    for (int f = 0; f < 4; ++f) load_vec<Dm>(W.rows + f * N, fields[f], e);
+  }
+  unsigned target = 0;
+  for (int it = 0; it < ns.nsteps; ++it) {
+    for (int st = 0; st < 4; ++st) {
+      const bool last = sa.stage < 0 || (it == ns.nsteps - 1 && st == 3);
+      const NlArgs &na = ns.nl;
+      if (active) {
+        const double *const in[2] = {st == 0 ? sa.base[0] : (st == 2 ? ns.bufb[0] : ns.bufa[0]),
+                                     st == 0 ? sa.base[1] : (st == 2 ? ns.bufb[1] : ns.bufa[1])};
+        // q-phase
+#pragma unroll
+        for (int c = 0; c < 2; ++c) reg_to_sm<Dm>(W.q.own + c * N, x[c]);
+        stage_neighbours<Dm, 2>(sd, W.q.nb, [&](int f, int t, int i) {
+          return __ldcg((f ? in[1] : in[0]) + (size_t)t * N + i);
+        });
+        __syncwarp();
+        double gq[4][R];
+        qphase_elem<Dm, VAR>(S, m, e, sd, W.q.own, W.q.nb, W.q.fr, W.q.fb, W.sm, [] {}, gq);
+        __syncwarp();
+        // quadrature-point phase
+#pragma unroll
+        for (int c = 0; c < 3; ++c) reg_to_sm<Dm>(W.b.rows + c * N, x[c]);
+        if (l < N) {
+#pragma unroll
+          for (int f = 0; f < 4; ++f) W.b.rows[(3 + f) * N + l] = W.rows[f * N + l];
+        }
+        __syncwarp();
+        nlvol_elem<Dm, VAR>(SQ, SQ.p2, SQ.p2t, SQ.wi, W.b.vin, W.b.wp, W.b.tail, W.sm, m, na, e, gq,
+                            W.b.rows, [] {});
+      }
+      target += gridDim.x;
+      if (!grid_barrier(ns.count, target, op.flag)) return;
+      if (active) {
+        const double *const src[6] = {na.f, na.f + fs, na.f + 2 * fs, na.f + 3 * fs, na.uh, na.vh};
+#pragma unroll
+        for (int f = 0; f < 6; ++f) load_vec<Dm>(W.t.own + f * N, src[f], e);
+        stage_neighbours<Dm, 6>(sd, W.t.nb,
+                                [&](int f, int t, int i) { return __ldcg(src[f] + (size_t)t * N + i); });
+        __syncwarp();
+        double d[3][R];
+        tend_elem<Dm, VAR>(
+            S, m, e, sd, W.t.own, W.t.nb, W.t.fb, W.sm,
+            [&](double(&gx)[R], double(&gy)[R]) {
+              load_reg<Dm>(gx, na.gx0, e);
+              load_reg<Dm>(gy, na.gy0, e);
+            },
+            [] {}, d[0], d[1], d[2]);
+        __syncwarp();
+        // stage_update with u0 and the accumulator in registers
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          double *const out = st == 1 ? ns.bufb[c] : ns.bufa[c];
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const int i = l + 32 * r;
+            if (i >= N) continue;
+            const size_t o = (size_t)e * N + i;
+            const double dd = d[c][r];
+            if (!isfinite(dd)) atomicOr(sa.flag, 1);
+            if (sa.stage < 0) {
+              sa.tend[c][o] = dd;
+            } else if (st == 3) {
+              const double nv = add(u0[c][r], mul(sa.dt6, add(acc[c][r], dd)));
+              u0[c][r] = x[c][r] = nv;
+              sa.base[c][o] = nv;
+              if (last && ns.host[c]) ns.host[c][(size_t)e * sa.host_ld + i] = nv;
+            } else {
+              acc[c][r] = st == 0 ? dd : add(acc[c][r], mul(2.0, dd));
+              const double s = mul(sa.dt, dd);
+              x[c][r] = add(u0[c][r], st == 2 ? s : mul(s, 0.5));
+              out[o] = x[c][r];
+            }
+          }
+        }
+        __syncwarp();
+      }
+      if (last) return;
+      target += gridDim.x;
+      if (!grid_barrier(ns.count, target, op.flag)) return;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
 // operator images: the shared-memory layouts of SOps / SOpsQ, written once per
 // handle into global memory so that each block stages them with bulk copies
 // ---------------------------------------------------------------------------
@@ -1924,6 +2089,56 @@ cudaError_t run_lin_steps(const DevOps &op, const DevMesh &m, const LinSteps &ls
   return e;
 }
 
+// The multi-step nonlinear kernel where a block per SM holds the mesh with one
+// element per warp (16 at most); else cudaErrorNotSupported.  Up to eight
+// warps a block the registers are left to the compiler, beyond that they are
+// held to 16 warps.  us per right-hand side of a run, five launches from the
+// step graph / here: degree 3 31 / 16 at 288 elements, 35 / 23 at 2312;
+// degree 4 41 / 29, 42 / 35; degree 5 56 / 36, 62 / 44; degree 6 59 / 45,
+// 77 / 58.  Degree 7 (two rows per lane) keeps the per-stage kernels: 67 / 73
+// at 288 elements, 107 / 108 at 1682.
+template <class Dm, int VAR>
+cudaError_t run_nl_steps(const DevOps &op, const DevMesh &m, const NlSteps &ns, cudaStream_t st, int sms,
+                         long long *launches) {
+  constexpr size_t ops = sizeof(SOps<Dm>) + sizeof(SOpsQ<Dm>);
+  constexpr int fit = (int)((226 * 1024 - ops) / sizeof(NWarp<Dm>));
+  constexpr int most = std::min(fit, 16);
+  if (m.ne < 1 || sms < 1) return cudaErrorNotSupported;
+  const int w = (m.ne + sms - 1) / sms;
+  if (w > most) return cudaErrorNotSupported;
+  const size_t sm = ops + w * sizeof(NWarp<Dm>);
+  const auto kern = w <= 8 ? kf_nl_steps<Dm, VAR, 8> : kf_nl_steps<Dm, VAR, 16>;
+  int per_sm = 0;
+  cudaError_t e = device_blocks_per_sm(kern, 32 * w, sm, &per_sm);
+  if (e == cudaErrorInvalidConfiguration) return cudaErrorNotSupported;  // no room on an SM
+  if (e != cudaSuccess) return e;
+  const int grid = (m.ne + w - 1) / w;  // <= sms blocks, one per SM
+  if (ns.nsteps <= 0) return cudaSuccess;
+  e = cudaMemsetAsync(ns.count, 0, sizeof(unsigned), st);
+  if (e != cudaSuccess) return e;
+  DevOps o = op;
+  DevMesh mm = m;
+  NlSteps n = ns;
+  void *args[] = {&o, &mm, &n};
+  e = cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(kern), dim3(grid), dim3(32 * w), args, sm,
+                                  st);
+  if (e == cudaSuccess) *launches += 1;
+  return e;
+}
+template <class Dm>
+cudaError_t run_nl_steps_any(int variant, const DevOps &op, const DevMesh &m, const NlSteps &ns,
+                             cudaStream_t st, int sms, long long *launches) {
+  if constexpr (Dm::R == 1) {
+    switch (variant) {
+      case kFS: return run_nl_steps<Dm, kFS>(op, m, ns, st, sms, launches);
+      case kNS: return run_nl_steps<Dm, kNS>(op, m, ns, st, sms, launches);
+      case kINV: return run_nl_steps<Dm, kINV>(op, m, ns, st, sms, launches);
+      default: break;
+    }
+  }
+  return cudaErrorNotSupported;
+}
+
 template <class Dm>
 cudaError_t run_lin(const DevOps &op, const DevMesh &m, const RhsBuffers &b, const StageArgs &sa,
                     cudaStream_t st, int sms, cudaEvent_t *ev) {
@@ -1958,10 +2173,12 @@ cudaError_t run_any(int variant, const DevOps &op, const DevMesh &m, const RhsBu
 #define FAST_AVAILABLE fast_available_fma
 #define LAUNCH_FAST launch_rhs_fast_fma
 #define LIN_STEPS_FAST lin_steps_fast_fma
+#define NL_STEPS_FAST nl_steps_fast_fma
 #else
 #define FAST_AVAILABLE fast_available
 #define LAUNCH_FAST launch_rhs_fast
 #define LIN_STEPS_FAST lin_steps_fast
+#define NL_STEPS_FAST nl_steps_fast
 #endif
 
 bool FAST_AVAILABLE(int nc, int ng, int ngf) {
@@ -2047,6 +2264,17 @@ cudaError_t LIN_STEPS_FAST(const DevOps &op, const DevMesh &m, const LinSteps &l
   if (nc == 5 && ng == 27 && ngf == 6) return run_lin_steps<Dims<5, 27, 6>>(op, m, ls, st, sms, launches);
   if (nc == 6 && ng == 33 && ngf == 7) return run_lin_steps<Dims<6, 33, 7>>(op, m, ls, st, sms, launches);
   if (nc == 7 && ng == 42 && ngf == 9) return run_lin_steps<Dims<7, 42, 9>>(op, m, ls, st, sms, launches);
+  return cudaErrorNotSupported;
+}
+
+cudaError_t NL_STEPS_FAST(int variant, const DevOps &op, const DevMesh &m, const NlSteps &ns,
+                          cudaStream_t st, int sms, long long *launches) {
+  const int nc = op.nc, ng = op.ng, ngf = op.ngf;
+  if (nc == 3 && ng == 12 && ngf == 4) return run_nl_steps_any<Dims<3, 12, 4>>(variant, op, m, ns, st, sms, launches);
+  if (nc == 4 && ng == 25 && ngf == 5) return run_nl_steps_any<Dims<4, 25, 5>>(variant, op, m, ns, st, sms, launches);
+  if (nc == 5 && ng == 27 && ngf == 6) return run_nl_steps_any<Dims<5, 27, 6>>(variant, op, m, ns, st, sms, launches);
+  if (nc == 6 && ng == 33 && ngf == 7) return run_nl_steps_any<Dims<6, 33, 7>>(variant, op, m, ns, st, sms, launches);
+  if (nc == 7 && ng == 42 && ngf == 9) return run_nl_steps_any<Dims<7, 42, 9>>(variant, op, m, ns, st, sms, launches);
   return cudaErrorNotSupported;
 }
 

@@ -59,6 +59,20 @@ struct LinSteps {
   int norder = 0;
 };
 
+// Several RK4 steps of a nonlinear variant (sa.stage >= 0), or one right-hand
+// side into sa.tend (sa.stage < 0, nsteps 1), in one launch: nl carries the
+// time-constant fields, the intermediates and the parameters (su, sv, sh, q
+// are not used); the rest as in LinSteps.
+struct NlSteps {
+  StageArgs sa;
+  NlArgs nl;
+  double *bufa[3];
+  double *bufb[3];
+  double *host[3];
+  int nsteps;
+  unsigned *count;
+};
+
 // Tangent-linear quadrature-point stage: base state (su.., q) and perturbation
 // (du, dv, dh, dq) in; perturbations of gx0, gy0, uh, vh, F out.
 struct TlmArgs {
@@ -237,7 +251,13 @@ cudaError_t launch_qphase_tile(int variant, const DevOps &op, const DevMesh &m, 
 cudaError_t lin_steps_fast(const DevOps &op, const DevMesh &m, const LinSteps &ls, cudaStream_t st,
                            int sms, long long *launches);
 
+// The same for the nonlinear variants: small meshes, one element per warp.
+cudaError_t nl_steps_fast(int variant, const DevOps &op, const DevMesh &m, const NlSteps &ns,
+                          cudaStream_t st, int sms, long long *launches);
+
 // The same kernels with fused multiply-adds (spoc_fast.cu built with SPOC_FMA=1).
+cudaError_t nl_steps_fast_fma(int variant, const DevOps &op, const DevMesh &m, const NlSteps &ns,
+                              cudaStream_t st, int sms, long long *launches);
 bool fast_available_fma(int nc, int ng, int ngf);
 cudaError_t launch_rhs_fast_fma(int variant, const DevOps &op, const DevMesh &m,
                                 const RhsBuffers &b, const StageArgs &sa, cudaStream_t st, int sms,

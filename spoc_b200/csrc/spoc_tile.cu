@@ -168,14 +168,14 @@ struct Degree {
   // elements per SM from which these kernels win over one element per warp
   // (spoc_fast.cu), whose 16 warps an SM take a second round near there: us
   // per right-hand side here / there 34 / 33 at 1152 elements and 35 / 38 at
-  // 2048 (degree 3); 41 / 45 at 288 (degree 4); 61 / 60 at 1152, 63 / 70 at
-  // 2048 (degree 5); 81 / 73 at 2048, 89 / 99 at 3200 (degree 6); 116 / 84 at
-  // 1152, 121 / 132 at 2048 (degree 7)
+  // 2048 (degree 3); 41 / 45 at 288, 42 / 54 at 2048 (degree 4); 61 / 60 at
+  // 1152, 63 / 70 at 2048 (degree 5); 81 / 73 at 2048, 89 / 99 at 3200 (degree
+  // 6); 116 / 84 at 1152, 121 / 132 at 2048 (degree 7)
   // linear variant (one kernel there, two here): 24 / 21 at 2048 elements and
   // 23 / 26 at 3200 (degree 4), 23 / 23 at 2048 (degree 5), 28 / 26 at 2048 and
   // 32 / 36 at 3200 (degree 6), 37 / 52 at 2048 (degree 7)
   static constexpr int MIN_PER_SM_LIN = 16;
-  static constexpr int MIN_PER_SM = NC == 4 ? 0 : (NC == 6 ? 17 : (NC == 7 ? 13 : 10));
+  static constexpr int MIN_PER_SM = NC == 6 ? 17 : (NC == 7 ? 13 : 10);
 };
 template <class P>
 struct Images {

@@ -1,7 +1,7 @@
 """Kernels with several elements per warp.  FP64 (spoc_tile.cu) against the
 CPU oracle, bit for bit: every tabulated degree and variant on a mesh
 large enough for them whose element and face counts are not multiples of a
-tile, the smallest meshes that reach them (degree 4), and an odd element count
+tile, and an odd element count
 at an odd mode count (fields aligned to 8 bytes only).  Mixed precision
 (spoc_mixed_tile.cu) against the one-element-per-warp kernels, which sum every
 chain in the same order: also bit for bit."""
@@ -67,18 +67,20 @@ def test_ragged_mesh_bitwise(gpu_lib, nc, variant):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("variant", ["fs", "ns"])
-@pytest.mark.parametrize("n", [2, 3])
-def test_smallest_meshes_bitwise(gpu_lib, n, variant):
-    check(problem(4, variant, n))
-
-
-@pytest.mark.gpu
-@pytest.mark.parametrize("nc,n", [(4, 4), (5, 37)])
+@pytest.mark.parametrize("nc,n", [(4, 35), (5, 37)])
 def test_odd_element_count_bitwise(gpu_lib, nc, n):
     p = problem(nc, "fs", n, odd=True)
     assert p.mesh.ne % 2 == 1
     check(p)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("variant", ["fs", "ns", "inv"])
+@pytest.mark.parametrize("nc,n", [(3, 2), (3, 34), (4, 13), (5, 9), (5, 25), (6, 2), (6, 24), (6, 34)])
+def test_small_mesh_one_launch_bitwise(gpu_lib, nc, n, variant):
+    """Small meshes: all steps of a call in one cooperative launch, with one
+    warp per block, the most of either instance, and idle warps."""
+    check(problem(nc, variant, n))
 
 
 @pytest.mark.gpu
