@@ -62,7 +62,10 @@ template <class T, int VAR, int W>
 __global__ void __launch_bounds__(32 * W, 1) kx_vol_tile(const MxArgs a) {
   extern __shared__ __align__(16) float sm[];
   __shared__ __align__(8) uint64_t bar;
-  if (!bulk::stage_block(sm, a.timg, sizeof(float) * T::NOPS, &bar, a.flag)) return;
+  grid_next();
+  const bool staged = bulk::stage_block(sm, a.timg, sizeof(float) * T::NOPS, &bar, a.flag);
+  grid_wait();
+  if (!staged) return;
   float *w = sm + T::NOPS + (threadIdx.x >> 5) * T::WS;
   const int step = gridDim.x * W;
   int t = blockIdx.x + gridDim.x * (threadIdx.x >> 5);
@@ -76,7 +79,10 @@ __global__ void __launch_bounds__(32 * W, 1) kx_tend_tile(const MxArgs a) {
   extern __shared__ __align__(16) float sm[];
   __shared__ __align__(8) uint64_t bar;
   constexpr int OPS = T::NOPS - T::TRT;
-  if (!bulk::stage_block(sm, a.timg + IMG + T::TRT, sizeof(float) * OPS, &bar, a.flag)) return;
+  grid_next();
+  const bool staged = bulk::stage_block(sm, a.timg + IMG + T::TRT, sizeof(float) * OPS, &bar, a.flag);
+  grid_wait();
+  if (!staged) return;
   float *w = sm + OPS + (threadIdx.x >> 5) * T::TWS;
   const int step = gridDim.x * W;
   int t = blockIdx.x + gridDim.x * (threadIdx.x >> 5);
@@ -89,12 +95,15 @@ constexpr int warps(int ops, int per_warp, int most) {
   return w < most ? w : most;
 }
 
-template <class K>
-cudaError_t launch(K k, int W, size_t smem, int sms, int tiles, const MxArgs &a, cudaStream_t st) {
+// chained: behind the kernel before it in the stream (launch_chained)
+cudaError_t launch(void (*k)(MxArgs), int W, size_t smem, int sms, int tiles, const MxArgs &a,
+                   cudaStream_t st, bool chained) {
   int per_sm = 0;
   const cudaError_t e = device_blocks_per_sm(k, 32 * W, smem, &per_sm);
   if (e != cudaSuccess) return e;
-  k<<<std::min(tiles, sms * per_sm), 32 * W, smem, st>>>(a);
+  const int grid = std::min(tiles, sms * per_sm);
+  if (chained) return launch_chained(k, grid, 32 * W, smem, st, a);
+  k<<<grid, 32 * W, smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -103,12 +112,13 @@ cudaError_t run(const MxArgs &a, int sms, cudaStream_t st, cudaEvent_t mid) {
   using V = typename P::V;
   using T = typename P::T;
   constexpr int WV = warps(V::NOPS, V::WS, P::WV), WT = warps(T::NOPS - T::TRT, T::TWS, P::WT);
+  const bool chained = !mid && chain_pays(a.ne, T::N, sms);
   cudaError_t e = launch(kx_vol_tile<V, VAR, WV>, WV, 4 * (size_t)(V::NOPS + WV * V::WS), sms,
-                         (a.ne + V::E - 1) / V::E, a, st);
+                         (a.ne + V::E - 1) / V::E, a, st, chained);
   if (e == cudaSuccess && mid) e = cudaEventRecord(mid, st);
   if (e == cudaSuccess)
     e = launch(kx_tend_tile<T, VAR, WT, V::NOPS>, WT, 4 * (size_t)(T::NOPS - T::TRT + WT * T::TWS), sms,
-               (a.ne + T::E - 1) / T::E, a, st);
+               (a.ne + T::E - 1) / T::E, a, st, chained);
   return e;
 }
 

@@ -692,6 +692,7 @@ __global__ void __launch_bounds__(32 * W) kt_faces(DevOps op, const OpsF<D> *img
   extern __shared__ __align__(16) unsigned char smem[];
   OpsF<D> &S = *reinterpret_cast<OpsF<D> *>(smem);
   FaceWarp<D, FB> &w = reinterpret_cast<FaceWarp<D, FB> *>(smem + sizeof(OpsF<D>))[threadIdx.x >> 5];
+  grid_next();
   __shared__ const double *fields[NF];
   if (threadIdx.x == 0) {
 #pragma unroll
@@ -727,17 +728,13 @@ __global__ void __launch_bounds__(32 * W) kt_faces(DevOps op, const OpsF<D> *img
       for (int i = 0; i < 2; ++i)
         copy_row<D>(buf + (q * FE + row + 8 * i) * D::SN, fields[FB * b + q] + (size_t)t[i] * N, part);
   };
-  Ids ids{};
-  if (tile < ntile) {
-    ids = load_ids(tile);
-    issue(ids.t[0], 0, w.buf[0]);
-  }
-  cp_commit();
+  Ids ids = load_ids(min(tile, ntile - 1));
   __shared__ __align__(8) uint64_t ops_bar;
-  if (!bulk::stage_block(&S, img, sizeof(OpsF<D>), &ops_bar, op.flag)) {
-    cp_wait<0>();
-    return;
-  }
+  const bool staged = bulk::stage_block(&S, img, sizeof(OpsF<D>), &ops_bar, op.flag);
+  grid_wait();
+  if (!staged) return;
+  if (tile < ntile) issue(ids.t[0], 0, w.buf[0]);
+  cp_commit();
   for (; tile < ntile; tile += step) {
     const int next = tile + step;
     const int f = min(tile * FE + le, m.nf - 1);
@@ -838,16 +835,16 @@ __global__ void __launch_bounds__(32 * W) kt_qphase(DevOps op, const OpsE<D> *im
   QWarp<D> &w = reinterpret_cast<QWarp<D> *>(smem + sizeof(OpsE<D>))[threadIdx.x >> 5];
   const Lane l = lane_of<D>();
   const int ntile = (m.ne + E - 1) / E;
+  grid_next();
   Tiles<W> tiles(sched);
   int tile = tiles.first();
-  if (tile < ntile)
-    issue_group<D>(w.buf, su, sv, tile * E, m.ne, fv, 2 * G, 0, face_of_lane<D>(m, tile));
-  cp_commit();
+  const int face0 = face_of_lane<D>(m, min(tile, ntile - 1));
   __shared__ __align__(8) uint64_t ops_bar;
-  if (!bulk::stage_block(&S, img, sizeof(OpsE<D>), &ops_bar, op.flag)) {
-    cp_wait<0>();
-    return;
-  }
+  const bool staged = bulk::stage_block(&S, img, sizeof(OpsE<D>), &ops_bar, op.flag);
+  grid_wait();
+  if (!staged) return;
+  if (tile < ntile) issue_group<D>(w.buf, su, sv, tile * E, m.ne, fv, 2 * G, 0, face0);
+  cp_commit();
   const size_t fs = (size_t)m.ne * N;
   for (int next; tile < ntile; tile = next) {
     tiles.ask();
@@ -993,8 +990,11 @@ __global__ void __launch_bounds__(32 * W) kt_nlvol(DevOps op, const OpsQ<D> *img
   extern __shared__ __align__(16) unsigned char smem[];
   OpsQ<D> &S = *reinterpret_cast<OpsQ<D> *>(smem);
   NWarp<D> &w = reinterpret_cast<NWarp<D> *>(smem + sizeof(OpsQ<D>))[threadIdx.x >> 5];
+  grid_next();
   __shared__ __align__(8) uint64_t ops_bar;
-  if (!bulk::stage_block(&S, img, sizeof(OpsQ<D>), &ops_bar, op.flag)) return;
+  const bool staged = bulk::stage_block(&S, img, sizeof(OpsQ<D>), &ops_bar, op.flag);
+  grid_wait();
+  if (!staged) return;
   const Lane l = lane_of<D>();
   const int ntile = (m.ne + E - 1) / E;
   const size_t fs = (size_t)m.ne * N;
@@ -1175,19 +1175,17 @@ __global__ void __launch_bounds__(32 * W) kt_tendency(DevOps op, const OpsE<D> *
     const double *f0 = grp < 2 ? a.f + 2 * grp * fs : a.uh, *f1 = grp < 2 ? f0 + fs : a.vh;
     issue_group<D>(buf, f0, f1, t * E, m.ne, a.fv, 6 * G, 2 * G * grp, face);
   };
-  int face = 0, nface = 0;  // of this lane's record, in this tile and the next
-  if (tile < ntile) {
-    face = face_of_lane<D>(m, tile);
-    issue(tile, face, 0, w.buf[0]);
-  }
+  grid_next();
+  // of this lane's record, in this tile and the next
+  int face = face_of_lane<D>(m, min(tile, ntile - 1)), nface = 0;
+  __shared__ __align__(8) uint64_t ops_bar;
+  const bool staged = bulk::stage_block(&S, img, sizeof(OpsE<D>), &ops_bar, op.flag);
+  grid_wait();
+  if (!staged) return;
+  if (tile < ntile) issue(tile, face, 0, w.buf[0]);
   cp_commit();
   if (tile < ntile) issue(tile, face, 1, w.buf[1]);
   cp_commit();
-  __shared__ __align__(8) uint64_t ops_bar;
-  if (!bulk::stage_block(&S, img, sizeof(OpsE<D>), &ops_bar, op.flag)) {
-    cp_wait<0>();
-    return;
-  }
   double *buf = w.buf[0], *other = w.buf[1];
   for (int next; tile < ntile; tile = next, face = nface) {
     tiles.ask();
@@ -1329,13 +1327,14 @@ __global__ void __launch_bounds__(32 * W) kt_linear(DevOps op, const OpsE<D> *im
       for (int i = 0; i < 2 * G / LR; ++i) cp16(d + 2 * (h + LR * i), fv + (size_t)face * 4 * G + 2 * (h + LR * i));
     }
   };
-  if (tile < ntile) issue(tile, face_of_lane<D>(m, tile));
-  cp_commit();
+  grid_next();
+  const int face0 = face_of_lane<D>(m, min(tile, ntile - 1));
   __shared__ __align__(8) uint64_t ops_bar;
-  if (!bulk::stage_block(&S, img, sizeof(OpsE<D>), &ops_bar, op.flag)) {
-    cp_wait<0>();
-    return;
-  }
+  const bool staged = bulk::stage_block(&S, img, sizeof(OpsE<D>), &ops_bar, op.flag);
+  grid_wait();
+  if (!staged) return;
+  if (tile < ntile) issue(tile, face0);
+  cp_commit();
   const double mg0 = -a.g0, hh0 = a.hh0;
   for (int next; tile < ntile; tile = next) {
     tiles.ask();
@@ -1455,43 +1454,40 @@ constexpr int warps(size_t ops, size_t per_warp, int most) {
   return w < most ? w : most;
 }
 
-template <class K>
-cudaError_t tile_grid(K kernel, int w, size_t smem, int sms, int tiles, int *grid) {
+// chained: behind the kernel before it in the stream (launch_chained)
+template <class... P, class... A>
+cudaError_t launch_tiles(void (*kernel)(P...), int w, size_t smem, int sms, int tiles, cudaStream_t st,
+                         bool chained, A... args) {
   int per_sm = 0;
   const cudaError_t e = device_blocks_per_sm(kernel, 32 * w, smem, &per_sm);
-  if (e == cudaSuccess) *grid = std::min(tiles, sms * per_sm);
-  return e;
+  if (e != cudaSuccess) return e;
+  const int grid = std::min(tiles, sms * per_sm);
+  if (chained) return launch_chained(kernel, grid, 32 * w, smem, st, args...);
+  kernel<<<grid, 32 * w, smem, st>>>(args...);
+  return cudaGetLastError();
 }
 
 template <class P, int NF, int FB>
 cudaError_t run_faces(const DevOps &op, const Images<P> *im, const DevMesh &m, const FaceArgs &fa,
-                      cudaStream_t st, int sms) {
+                      cudaStream_t st, int sms, bool chained) {
   using D = typename P::DQ;
   constexpr int W = warps(sizeof(OpsF<D>), sizeof(FaceWarp<D, FB>), 16);
   constexpr size_t sm = sizeof(OpsF<D>) + W * sizeof(FaceWarp<D, FB>);
-  const auto k = kt_faces<D, NF, FB, W>;
-  int grid = 0;
-  const cudaError_t e = tile_grid(k, W, sm, sms, (m.nf + FE - 1) / FE, &grid);
-  if (e != cudaSuccess) return e;
-  k<<<grid, 32 * W, sm, st>>>(op, &im->f, m, fa);
-  return cudaGetLastError();
+  return launch_tiles(kt_faces<D, NF, FB, W>, W, sm, sms, (m.nf + FE - 1) / FE, st, chained, op, &im->f,
+                      m, fa);
 }
 
 template <class P, int VAR>
 cudaError_t run_q(const DevOps &op, const Images<P> *im, const DevMesh &m, const double *su,
-                  const double *sv, double *q, double *fv, cudaStream_t st, int sms) {
+                  const double *sv, double *q, double *fv, cudaStream_t st, int sms, bool chained) {
   const FaceArgs fa{{su, sv}, fv};
   using D = typename P::DQ;
-  cudaError_t e = run_faces<P, 2, 2>(op, im, m, fa, st, sms);
+  cudaError_t e = run_faces<P, 2, 2>(op, im, m, fa, st, sms, chained);
   if (e != cudaSuccess) return e;
   constexpr int W = warps(sizeof(OpsE<D>), sizeof(QWarp<D>), P::WQ);
   constexpr size_t sm = sizeof(OpsE<D>) + W * sizeof(QWarp<D>);
-  const auto k = kt_qphase<D, VAR, W>;
-  int grid = 0;
-  e = tile_grid(k, W, sm, sms, (m.ne + D::E - 1) / D::E, &grid);
-  if (e != cudaSuccess) return e;
-  k<<<grid, 32 * W, sm, st>>>(op, &im->e, m, su, sv, q, fv, op.sched);
-  return cudaGetLastError();
+  return launch_tiles(kt_qphase<D, VAR, W>, W, sm, sms, (m.ne + D::E - 1) / D::E, st, chained, op, &im->e, m,
+                      su, sv, q, fv, op.sched);
 }
 
 template <class P, int VAR>
@@ -1501,8 +1497,11 @@ cudaError_t run_nl(const DevOps &op, const DevMesh &m, const RhsBuffers &b, cons
   auto mark = [&](int i) {
     if (ev) cudaEventRecord(ev[i], st);
   };
+  // (timing events between the kernels, and the wait for h's upload, want them
+  // one after the other)
+  const bool chained = !ev && chain_pays(m.ne, P::DT::N, sms);
   mark(0);
-  cudaError_t e = run_q<P, VAR>(op, im, m, b.su, b.sv, b.q, b.fv, st, sms);
+  cudaError_t e = run_q<P, VAR>(op, im, m, b.su, b.sv, b.q, b.fv, st, sms, chained);
   if (e == cudaSuccess && b.sh_ready) e = cudaStreamWaitEvent(st, b.sh_ready, 0);
   if (e != cudaSuccess) return e;
   mark(1);
@@ -1512,29 +1511,23 @@ cudaError_t run_nl(const DevOps &op, const DevMesh &m, const RhsBuffers &b, cons
                     b.mu0, b.mb0, b.g0};
     constexpr int W = warps(sizeof(OpsQ<D>), sizeof(NWarp<D>), P::WV);
     constexpr size_t sm = sizeof(OpsQ<D>) + W * sizeof(NWarp<D>);
-    const auto k = kt_nlvol<D, VAR, W>;
-    int grid = 0;
-    e = tile_grid(k, W, sm, sms, (m.ne + D::E - 1) / D::E, &grid);
+    e = launch_tiles(kt_nlvol<D, VAR, W>, W, sm, sms, (m.ne + D::E - 1) / D::E, st, chained && !b.sh_ready, op,
+                     &im->q, m, na, op.sched + 2);
     if (e != cudaSuccess) return e;
-    k<<<grid, 32 * W, sm, st>>>(op, &im->q, m, na, op.sched + 2);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   mark(2);
   const size_t fs = (size_t)m.ne * P::DT::N;
   const FaceArgs fa{{b.f, b.f + fs, b.f + 2 * fs, b.f + 3 * fs, b.uh, b.vh}, b.fv};
-  e = run_faces<P, 6, P::FB>(op, im, m, fa, st, sms);
+  e = run_faces<P, 6, P::FB>(op, im, m, fa, st, sms, chained);
   if (e != cudaSuccess) return e;
   {
     using D = typename P::DT;
     const TendArgs ta{b.gx0, b.gy0, b.uh, b.vh, b.f, b.fv};
     constexpr int W = warps(sizeof(OpsE<D>), sizeof(TWarp<D>), P::WT);
     constexpr size_t sm = sizeof(OpsE<D>) + W * sizeof(TWarp<D>);
-    const auto k = kt_tendency<D, VAR, W>;
-    int grid = 0;
-    e = tile_grid(k, W, sm, sms, (m.ne + D::E - 1) / D::E, &grid);
+    e = launch_tiles(kt_tendency<D, VAR, W>, W, sm, sms, (m.ne + D::E - 1) / D::E, st, chained, op, &im->t, m, ta,
+                     sa, op.sched + 4);
     if (e != cudaSuccess) return e;
-    k<<<grid, 32 * W, sm, st>>>(op, &im->t, m, ta, sa, op.sched + 4);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   mark(3);
   *launches += 5;
@@ -1548,18 +1541,15 @@ cudaError_t run_lin(const DevOps &op, const DevMesh &m, const RhsBuffers &b, con
   const Images<P> *im = static_cast<const Images<P> *>(op.img_tile);
   cudaError_t e = b.sh_ready ? cudaStreamWaitEvent(st, b.sh_ready, 0) : cudaSuccess;
   if (ev && e == cudaSuccess) e = cudaEventRecord(ev[0], st);
+  const bool chained = !ev && chain_pays(m.ne, P::DT::N, sms);
   const FaceArgs fa{{b.sh, b.su, b.sv}, b.fv, -b.g0};
-  if (e == cudaSuccess) e = run_faces<P, 3, 3>(op, im, m, fa, st, sms);
+  if (e == cudaSuccess) e = run_faces<P, 3, 3>(op, im, m, fa, st, sms, chained && !b.sh_ready);
   if (e != cudaSuccess) return e;
   constexpr int W = warps(sizeof(OpsE<D>), sizeof(LWarp<D>), 12);
   constexpr size_t sm = sizeof(OpsE<D>) + W * sizeof(LWarp<D>);
-  const auto k = kt_linear<D, W>;
-  int grid = 0;
-  e = tile_grid(k, W, sm, sms, (m.ne + D::E - 1) / D::E, &grid);
-  if (e != cudaSuccess) return e;
   const LinArgs la{b.su, b.sv, b.sh, b.g0, b.hh0};
-  k<<<grid, 32 * W, sm, st>>>(op, &im->t, m, la, b.fv, sa, op.sched + 4);
-  e = cudaGetLastError();
+  e = launch_tiles(kt_linear<D, W>, W, sm, sms, (m.ne + D::E - 1) / D::E, st, chained, op, &im->t, m, la, b.fv, sa,
+                   op.sched + 4);
   if (ev && e == cudaSuccess) e = cudaEventRecord(ev[1], st);
   *launches += 2;
   return e;
@@ -1616,8 +1606,8 @@ cudaError_t launch_qphase_tile(int variant, const DevOps &op, const DevMesh &m, 
     using P = decltype(d);
     const Images<P> *im = static_cast<const Images<P> *>(op.img_tile);
     // the wall projection of the gradients is the free-slip variant's alone
-    if (variant == kFS) e = run_q<P, kFS>(op, im, m, su, sv, q, fv, st, sms);
-    else if (variant != kLIN) e = run_q<P, kINV>(op, im, m, su, sv, q, fv, st, sms);
+    if (variant == kFS) e = run_q<P, kFS>(op, im, m, su, sv, q, fv, st, sms, chain_pays(m.ne, P::DQ::N, sms));
+    else if (variant != kLIN) e = run_q<P, kINV>(op, im, m, su, sv, q, fv, st, sms, chain_pays(m.ne, P::DQ::N, sms));
   });
   return e;
 }
