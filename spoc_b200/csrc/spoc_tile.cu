@@ -50,6 +50,24 @@ __device__ __forceinline__ double macc(double acc, double a, double b) { return 
 __device__ __forceinline__ double msub(double acc, double a, double b) { return sub(acc, mul(a, b)); }
 #endif
 
+// acc(i) += x(i) y(i) for i < K.  B: all products first.  ptxas keeps a product
+// and its add close together, and a batch spreads them: degree 7 696 -> 672 us
+// per right-hand side, degree 6 417 -> 413; at smaller degrees, with more warps
+// to fill the gaps, the registers it takes cost more (degree 5 282 -> 286).
+template <bool B, int K, class A, class X, class Y>
+__device__ __forceinline__ void maccs(A acc, X x, Y y) {
+  if constexpr (B && !SPOC_FMA) {
+    double t[K];
+#pragma unroll
+    for (int i = 0; i < K; ++i) t[i] = mul(x(i), y(i));
+#pragma unroll
+    for (int i = 0; i < K; ++i) acc(i) = add(acc(i), t[i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < K; ++i) acc(i) = macc(acc(i), x(i), y(i));
+  }
+}
+
 constexpr int FE = 16;  // faces per warp of the face-value kernel
 constexpr int FG = 2;   // point groups per face
 __host__ __device__ constexpr int even(int n) { return n + (n & 1); }
@@ -65,6 +83,7 @@ struct Dims {
   static constexpr int RN = (N + RG - 1) / RG;   // modal rows per thread
   static constexpr int RM = (M + RG - 1) / RG;
   static constexpr int CW = even(RN) * RG;       // operator column, rows dealt and padded
+  static constexpr bool BATCH = N >= 28;         // products in batches (maccs)
   // stride of an element's coefficients in shared memory: 16-byte pairs of
   // eight elements in eight bank groups (even N), or odd (8-byte loads)
   static constexpr int SN = (N % 2) ? N : ((N / 2) % 2 ? N : N + 2);
@@ -498,16 +517,15 @@ __device__ __forceinline__ void matvec2(const double *A, const double *B, const 
 #pragma unroll
     for (int p = 0; p < (RN + 1) / 2; ++p) {
       const double2 va = ld2(pa + p * 2 * RG), vb = ld2(pb + p * 2 * RG);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int r = 2 * p + h;
-        if (r >= RN) continue;
-        const double oa = h ? va.y : va.x, ob = h ? vb.y : vb.x;
-        a[0][r] = macc(a[0][r], oa, c0);
-        b[0][r] = macc(b[0][r], ob, c0);
-        a[1][r] = macc(a[1][r], oa, c1);
-        b[1][r] = macc(b[1][r], ob, c1);
-      }
+      // i = 4 (row of the pair) + 2 (field) + operator
+      auto rows = [&](auto n) {
+        maccs<D::BATCH, 4 * decltype(n)::value>(
+            [&](int i) -> double & { return (i & 1 ? b : a)[(i >> 1) & 1][2 * p + (i >> 2)]; },
+            [&](int i) { return i & 1 ? (i >> 2 ? vb.y : vb.x) : (i >> 2 ? va.y : va.x); },
+            [&](int i) { return (i >> 1) & 1 ? c1 : c0; });
+      };
+      if (2 * p + 1 < RN) rows(std::integral_constant<int, 2>{});
+      else rows(std::integral_constant<int, 1>{});
     }
   };
   if constexpr (N % 2 == 0) {
@@ -1068,8 +1086,8 @@ __global__ void __launch_bounds__(32 * W) kt_nlvol(DevOps op, const OpsQ<D> *img
         for (int r = 0; r < PP; ++r) p[r] = p2[n * D::NP * QP + RG * r];
 #pragma unroll
         for (int r = 0; r < PP; ++r)
-#pragma unroll
-          for (int f = 0; f < 9; ++f) mv[r][f] = macc(mv[r][f], c[f], p[r]);
+          maccs<D::BATCH, 9>([&](int f) -> double & { return mv[r][f]; }, [&](int f) { return c[f]; },
+                             [&](int) { return p[r]; });
       }
 #pragma unroll
       for (int r = 0; r < PP; ++r) {
@@ -1103,8 +1121,8 @@ __global__ void __launch_bounds__(32 * W) kt_nlvol(DevOps op, const OpsQ<D> *img
           for (int h = 0; h < 2; ++h) {
             const int r = 2 * p + h;
             if (r >= RN) continue;
-#pragma unroll
-            for (int f = 0; f < 8; ++f) X[f][r] = macc(X[f][r], c[f], h ? v.y : v.x);
+            maccs<D::BATCH, 8>([&](int f) -> double & { return X[f][r]; }, [&](int f) { return c[f]; },
+                               [&](int) { return h ? v.y : v.x; });
           }
         }
       }
