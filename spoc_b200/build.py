@@ -26,14 +26,14 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC,-ffp-contract=off,-O2",
     "-Xptxas", "-v",
 ]
-SOURCES = ["spoc_tile.cu", "spoc_kernels.cu", "spoc_fast.cu", "spoc_api.cu", "spoc_noalloc.cu", "spoc_adjoint.cu",
+SOURCES = ["spoc_tile.cu", "spoc_kernels.cu", "spoc_fast.cu", "spoc_api.cu", "spoc_noalloc.cu", "spoc_adjoint.cu", "spoc_adjoint_tile.cu",
            "spoc_mixed.cu", "spoc_mixed_tile.cu", "spoc_mixed_tc.cu", "spoc_tc_selftest.cu", "spoc_regrid.cu"]
 # these are compiled a second time with fused multiply-adds
 VARIANT_SOURCES = [("spoc_fast.cu", "spoc_fast_fma", ["-DSPOC_FMA=1"]),
                    ("spoc_tile.cu", "spoc_tile_fma", ["-DSPOC_FMA=1"])]
 HOST_SOURCES = ["spoc_host.cpp"]
 HEADERS = ["spoc_device.cuh", "spoc_kernels.h", "spoc_launch.h", "spoc_bulk.cuh", "spoc_mixed.h", "spoc_tc.cuh",
-           "spoc_mixed_dev.cuh", "spoc_mixed_tile.cuh"]
+           "spoc_mixed_dev.cuh", "spoc_mixed_tile.cuh", "spoc_tile.cuh"]
 
 
 def _nvcc() -> str:

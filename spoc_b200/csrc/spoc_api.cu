@@ -1369,6 +1369,7 @@ struct AdjCtx {
          *aq = nullptr, *lx = nullptr, *ly = nullptr, *lh = nullptr, *lq = nullptr;
   // RK4 step work: states x, s2, s3, s4 (3 fields each), tendencies, vectors
   double *S[4][3] = {}, *K[4][3] = {}, *V[6][3] = {};
+  char *img = nullptr;  // operator images of the several-element kernels, where they run
   double *qs[3] = {};  // q of the forward stages 1-3 of the step being reversed
   // observations
   int nobs = 0, ntimes = 0, nel = 0;
@@ -1435,6 +1436,10 @@ int adj_init(spoc_handle *h, AdjCtx *c) {
     }
   for (int i = 0; i < 6; ++i)
     for (int f = 0; f < 3; ++f) A(&c->V[i][f], n);
+  if (h->variant != SPOC_LIN && h->op.img_tile && e == cudaSuccess) {
+    e = h->alloc(&c->img, adj_tile_image_bytes(h->nc, h->ng, h->ngf));
+    if (e == cudaSuccess) e = adj_tile_build_images(h->op, c->img, h->st);
+  }
   if (e != cudaSuccess) return fail(SPOC_E_NOMEM, "adjoint work space", e);
   c->ready = 1;
   return SPOC_OK;
@@ -1497,7 +1502,10 @@ int adj_rhs(spoc_handle *h, AdjCtx *c, double *const s[3], double *const b[3],
   AdjNlArgs na{s[0], s[1], s[2], h->hb, h->w0, h->z0, h->fc, qb, c->af, c->agx0, c->agy0,
                c->auh, c->avh, out[0], out[1], out[2], c->aq, h->mu0, h->mb0, h->g0};
   AdjQArgs qa{c->aq, out[0], out[1], c->lq};
-  CK(launch_adj_nl(h->variant, h->op, h->mesh, ta, na, qa, h->st, h->sms), "adjoint");
+  CK(c->img && h->path != SPOC_PATH_GENERIC
+         ? launch_adj_nl_tile(h->variant, h->op, c->img, h->mesh, ta, na, qa, h->st, h->sms)
+         : launch_adj_nl(h->variant, h->op, h->mesh, ta, na, qa, h->st, h->sms),
+     "adjoint");
   return SPOC_OK;
 }
 

@@ -154,6 +154,14 @@ cudaError_t launch_nlvol_tlm(int variant, const DevOps &op, const DevMesh &m, co
                              cudaStream_t st, int sms);
 cudaError_t launch_adj_nl(int variant, const DevOps &op, const DevMesh &m, const AdjTendArgs &ta,
                           const AdjNlArgs &na, const AdjQArgs &qa, cudaStream_t st, int sms);
+// The same for the tabulated degrees with several elements per warp
+// (spoc_adjoint_tile.cu), the bytes of its operator images and the kernel that
+// writes them; identical results.
+size_t adj_tile_image_bytes(int nc, int ng, int ngf);
+cudaError_t adj_tile_build_images(const DevOps &op, void *img, cudaStream_t st);
+cudaError_t launch_adj_nl_tile(int variant, const DevOps &op, const void *img, const DevMesh &m,
+                               const AdjTendArgs &ta, const AdjNlArgs &na, const AdjQArgs &qa,
+                               cudaStream_t st, int sms);
 cudaError_t launch_adj_lin(const DevOps &op, const DevMesh &m, const AdjLinArgs &a,
                            cudaStream_t st, int sms);
 cudaError_t launch_axpy(size_t n, const double *x, double c, const double *y, double *out,

@@ -100,3 +100,21 @@ def test_mixed_ragged_mesh_matches_one_element_kernels(gpu_lib, nc, variant):
         out.append([*rhs, *s.get_state()])
     for a, b in zip(*out):
         assert np.isfinite(a).all() and np.array_equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("variant", ["fs", "ns", "inv"])
+@pytest.mark.parametrize("nc", sorted(RULES))
+def test_adjoint_ragged_mesh_matches_one_element_kernels(gpu_lib, nc, variant):
+    """Adjoint right-hand side and steps (spoc_adjoint_tile.cu) against
+    spoc_adjoint.cu, which sums in the same order: bit for bit."""
+    p = problem(nc, variant, 37)
+    x = [0.1 * f for f in (p.u, p.v, p.h)]
+    b = [np.random.default_rng(nc).normal(size=p.u.shape) for _ in range(3)]
+    out = []
+    for path in ("auto", "generic"):
+        s = W.make_solver(p)
+        s.set_kernel_path(path)
+        out.append([*s.adj_rhs(x, b), *s.adj_steps(x, b, 1.0e-3, 2)])
+    for g, r in zip(*out):
+        assert np.isfinite(g).all() and np.array_equal(g, r), f"max |d| = {np.abs(g - r).max():.3e}"
