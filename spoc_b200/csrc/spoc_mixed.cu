@@ -1284,6 +1284,7 @@ struct MixedEns {
   int sms = 148, bps = 0, weight = 0, nblk = 0, max_bps = 1;
   EnsMember *d_mem = nullptr;
   int *d_blk = nullptr;
+  unsigned *d_cnt = nullptr;  // tiles taken of each member in a phase
   unsigned long long *d_bt = nullptr;  // block cycles while balancing
   cudaStream_t st = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -1292,6 +1293,7 @@ struct MixedEns {
     if (exec) cudaGraphExecDestroy(exec);
     cudaFree(d_mem);
     cudaFree(d_blk);
+    cudaFree(d_cnt);
     cudaFree(d_bt);
     if (st) cudaStreamDestroy(st);
   }
@@ -1360,10 +1362,11 @@ int ens_layout(MixedEns *e) {
 
 cudaError_t ens_launch_step(MixedEns *e, int cur0, unsigned long long *bt = nullptr) {
   const EnsKernel k = mixed_tile_ens();
+  int n = (int)e->mem.size();
   for (int s = 0; s < 4; ++s) {
     int stage = s, cur = (cur0 + s) & 1;
-    void *args[] = {(void *)&e->d_mem, (void *)&e->d_blk, (void *)&stage, (void *)&cur,
-                    (void *)&bt};
+    void *args[] = {(void *)&e->d_mem, (void *)&e->d_blk, (void *)&n, (void *)&stage, (void *)&cur,
+                    (void *)&e->d_cnt, (void *)&bt};
     cudaError_t ce = cudaLaunchCooperativeKernel(k.kernel, dim3(e->nblk), dim3(k.threads), args,
                                                  k.smem, e->st);
     if (ce != cudaSuccess) return ce;
@@ -1402,6 +1405,8 @@ int mixed_ens_create(MixedEns **out, MixedCtx *const *ctx, const DevMesh *meshes
   if (ce == cudaSuccess)
     ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.kernel, k.threads, k.smem);
   if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking);
+  if (ce == cudaSuccess) ce = cudaMalloc(&e->d_cnt, 2 * sizeof(unsigned) * n);
+  if (ce == cudaSuccess) ce = cudaMemset(e->d_cnt, 0, 2 * sizeof(unsigned) * n);
   if (ce != cudaSuccess || occ < 1) {
     if (err) *err = std::string("ensemble set-up: ") + cudaGetErrorString(ce);
     delete e;

@@ -191,8 +191,9 @@ cudaError_t mixed_tc_tend(int variant, int nc, int ng, int ngf, const mx::MxArgs
 bool mixed_tile_pays(int nc, int ng, int ngf, int ne, int sms);
 std::vector<float> mixed_tile_image(int nc, int ng, int ngf, const PsiOps &p, const double *wi,
                                     const double *wif);
-// The ensemble kernel (EnsMember *, int *block member, int stage, int current
-// trace buffer, unsigned long long *block cycles), threads and shared memory.
+// The ensemble kernel (EnsMember *, int *block member, int members, int stage,
+// int current trace buffer, unsigned *tile counters, unsigned long long *block
+// cycles), threads and shared memory.
 struct EnsKernel {
   const void *kernel;
   int threads;

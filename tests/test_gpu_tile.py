@@ -118,3 +118,25 @@ def test_adjoint_ragged_mesh_matches_one_element_kernels(gpu_lib, nc, variant):
         out.append([*s.adj_rhs(x, b), *s.adj_steps(x, b, 1.0e-3, 2)])
     for g, r in zip(*out):
         assert np.isfinite(g).all() and np.array_equal(g, r), f"max |d| = {np.abs(g - r).max():.3e}"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("weight", [0, 3])
+def test_ensemble_blocks_help_other_members(gpu_lib, weight):
+    """One block per SM for members whose tiles exceed a first round, dealt so
+    that some members' blocks finish early and take other members' tiles."""
+    ps = [problem(nc, "fs", n) for nc, n in ((3, 50), (6, 41), (4, 13), (5, 60))]
+    alone, mem = [], []
+    for p in ps:
+        p.u, p.v, p.h = 0.1 * p.u, 0.1 * p.v, 0.1 * p.h
+        for out in (alone, mem):
+            out.append(W.make_solver(p, "mixed"))
+            out[-1].set_state(p.u, p.v, p.h)
+    for s in alone:
+        s.rk4_steps(1.0e-3, 3)
+    ens = api.Ensemble(mem)
+    ens.configure(1, weight)
+    ens.steps([1.0e-3] * len(ps), 3)
+    for a, b in zip(alone, mem):
+        for x, y in zip(a.get_state(), b.get_state()):
+            assert np.isfinite(x).all() and np.array_equal(x, y)
