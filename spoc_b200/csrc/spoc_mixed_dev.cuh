@@ -143,21 +143,23 @@ __device__ __forceinline__ float face_value(const float *tr, const FaceRef &r, i
                  (nb[TG * FS] - tr[((size_t)e * TS + TG) * FS]));
 }
 
-// RK4 bookkeeping of src/shwwnl.f:242-284 on one psi coefficient, FP64;
-// returns the next stage input.
-__device__ __forceinline__ double rk4_update(const MxArgs &a, size_t i, double d) {
-  double *c = a.c64 + i, *acc = a.acc + i;
-  const double u0 = *c;
+// RK4 bookkeeping of src/shwwnl.f:242-284 on one psi coefficient, FP64, from
+// its base value u0 and accumulator s (not read at stage 0); returns the next
+// stage input.
+__device__ __forceinline__ double rk4_update(const MxArgs &a, size_t i, double d, double u0, double s) {
   switch (a.stage) {
-    case 0: *acc = d; return u0 + a.dt * d * 0.5;
-    case 1: *acc = *acc + 2.0 * d; return u0 + a.dt * d * 0.5;
-    case 2: *acc = *acc + 2.0 * d; return u0 + a.dt * d;
+    case 0: a.acc[i] = d; return u0 + a.dt * d * 0.5;
+    case 1: a.acc[i] = s + 2.0 * d; return u0 + a.dt * d * 0.5;
+    case 2: a.acc[i] = s + 2.0 * d; return u0 + a.dt * d;
     default: {
-      const double u1 = u0 + a.dt6 * (*acc + d);
-      *c = u1;
+      const double u1 = u0 + a.dt6 * (s + d);
+      a.c64[i] = u1;
       return u1;
     }
   }
+}
+__device__ __forceinline__ double rk4_update(const MxArgs &a, size_t i, double d) {
+  return rk4_update(a, i, d, a.c64[i], a.stage > 0 ? a.acc[i] : 0.0);
 }
 
 // A member of an ensemble as its kernel sees it: the kernel's arguments (stage,

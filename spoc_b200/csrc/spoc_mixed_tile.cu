@@ -18,14 +18,15 @@ namespace {
 // 32768 triangles, us per launch (one element per warp: spoc_mixed.cu):
 // volume work with eight / four elements a warp (one) 24 / 27 (35) at degree
 // 3, 37 / 39 (67), 48 / 53 (115), 68 / 71 (134), 108 / 101 (200) at degree 7;
-// tendencies with four / eight 21 / 22 (25), 27 / 31 (27), 33 / 38 (41),
-// 44 / 51 (49), 54 / 67 (76).  (Two elements per thread, 16 a warp, halve the
+// tendencies with four 20 (25), 26 (27), 30 (41), 36 (49), 44 (76), with eight
+// a twentieth to a quarter more; twenty warps, sixteen cost 39 us and
+// twenty-four 41 at degree 6.  (Two elements per thread, 16 a warp, halve the
 // operator loads once more but leave 6 to 8 warps an SM: 79 us at degree 6.)
 template <int NC, int Q, int G>
 struct Degree {
   using V = TDims<NC, Q, G, NC == 7 ? 4 : 8>;
   using T = TDims<NC, Q, G, 4>;
-  static constexpr int WV = 16, WT = NC == 7 ? 32 : 20;
+  static constexpr int WV = 16, WT = 20;
   // elements per SM from which they win over one element per warp, us per
   // right-hand side here / there: 15.5 / 14.4 at 2048 elements and 16.1 / 16.5
   // at 3200 (degree 3); 19 / 21 at 288 (degree 4); 24.7 / 20.6 at 2048, 24.7 /
