@@ -6,13 +6,16 @@
 // fused multiply-add of a solve or a lift asks for an operator load of its own
 // and the load unit bounds them; here a 16-byte operator load feeds 4 to 18.
 // Us per adjoint right-hand side (no-slip, 32768 triangles) there / here:
-// degree 3 235 / 137, 4 348 / 210, 5 766 / 309, 6 1076 / 455, 7 3759 / 649; the
-// largest at degree 4 are the quadrature-point kernel (119 / 78) and the two
-// with solves (143 / 70).  On the smallest meshes that take the several-element
-// kernels (10 to 17 elements per SM): 59 / 49, 75 / 65, 92 / 90, 156 / 102,
-// 484 / 146, so both follow one rule.  What bounds them now is the latency of
-// the solves' column chains and of the element loads at 12 warps an SM; the
-// FP64 pipe and the memory are each busy for about a third of the time.
+// degree 3 235 / 118, 4 348 / 181, 5 766 / 245, 6 1076 / 392, 7 3759 / 557; the
+// largest at degree 4 are the quadrature-point kernel (119 / 72) and the two
+// with solves (143 / 66).  On the smallest meshes that take the several-element
+// kernels (10 to 17 elements per SM) these were ahead as well: 59 / 49, 75 / 65,
+// 92 / 90, 156 / 102, 484 / 146, so both follow one rule.  By count the FP64 pipe
+// and the memory each need about a quarter of the time at degree 4: what is left
+// is the latency of the solves' column chains and of the element loads at 12
+// warps an SM.  Rows that are read, added to and written back are all read
+// before the first store (the compiler keeps a load behind the stores before
+// it): the two face kernels 64 -> 43 us, the whole 210 -> 181.
 #include "spoc_tile.cuh"
 
 namespace spoc {
@@ -46,7 +49,8 @@ struct AdjDegree {
   using DA = Dims<NC, Q, G, NC <= 5 ? 8 : 4>;
   // two points a thread leave the registers and the shared memory for twelve
   // warps: 102 against 110 (four points) and 114 us (four points, eight
-  // warps) at degree 5, 183 against 200 (three) at degree 6, level elsewhere
+  // warps) at degree 5, 183 against 200 (three) at degree 6, level elsewhere (93
+  // and 169 us with the result rows loaded together)
   using DV = Dims<NC, Q, G, 4, 2>;
 };
 template <class P>
@@ -271,14 +275,17 @@ __global__ void __launch_bounds__(32 * W) ka_qphase(DevOps op, const OpsA<D> *im
     clear(y);
     rows_times<D, 2, RN, D::CW>(S.ax, w.x, 2 * X, x, l);
     rows_times<D, 2, RN, D::CW>(S.ay, w.x + X, 2 * X, y, l);
-    if (live) {
+    double ub[RN], vb[RN];
+    load_rows<D>(ub, a.ub, e, l);
+    load_rows<D>(vb, a.vb, e, l);
 #pragma unroll
-      for (int r = 0; r < RN; ++r) {
-        const size_t i = (size_t)e * N + D::RG * r + l.s;
-        if (D::RG * r + l.s >= N) continue;
-        a.ub[i] = a.ub[i] + -(x[0][r] + y[0][r]);
-        a.vb[i] = a.vb[i] + -(x[1][r] + y[1][r]);
-      }
+    for (int r = 0; r < RN; ++r) {
+      ub[r] = ub[r] + -(x[0][r] + y[0][r]);
+      vb[r] = vb[r] + -(x[1][r] + y[1][r]);
+    }
+    if (live) {
+      store_rows<D>(a.ub, ub, e, l);
+      store_rows<D>(a.vb, vb, e, l);
     }
     __syncwarp();
 #pragma unroll
@@ -374,21 +381,28 @@ __global__ void __launch_bounds__(32 * W) ka_faces(DevOps op, const OpsT<D> *img
         }
       }
     }
+    constexpr int NF = NL == 3 ? 6 : 2;
+    double *out[NF];
+    if constexpr (NL == 3) {
+#pragma unroll
+      for (int f = 0; f < 4; ++f) out[f] = a.fb + f * fs;
+      out[4] = a.uhb;
+      out[5] = a.vhb;
+    } else {
+      out[0] = a.ub;
+      out[1] = a.vb;
+    }
+    double x[NF][RN];
+#pragma unroll
+    for (int f = 0; f < NF; ++f) load_rows<D>(x[f], out[f], e, l);
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+      for (int r = 0; r < RN; ++r)
+        x[f][r] = x[f][r] + (NL == 3 ? o[f][r] : o[2 * f % NO][r] + o[(2 * f + 1) % NO][r]);
     if (live) {
 #pragma unroll
-      for (int r = 0; r < RN; ++r) {
-        const size_t i = (size_t)e * N + RG * r + l.s;
-        if (RG * r + l.s >= N) continue;
-        if constexpr (NL == 3) {
-#pragma unroll
-          for (int f = 0; f < 4; ++f) a.fb[f * fs + i] = a.fb[f * fs + i] + o[f][r];
-          a.uhb[i] = a.uhb[i] + o[4][r];
-          a.vhb[i] = a.vhb[i] + o[NO - 1][r];
-        } else {
-          a.ub[i] = a.ub[i] + (o[0][r] + o[1][r]);
-          a.vb[i] = a.vb[i] + (o[2][r] + o[3][r]);
-        }
-      }
+      for (int f = 0; f < NF; ++f) store_rows<D>(out[f], x[f], e, l);
     }
     __syncwarp();
   }
@@ -527,18 +541,20 @@ __global__ void __launch_bounds__(32 * W) ka_nlvol(DevOps op, const OpsQ<D> *img
     const int e = tile * E + p.e;
     if (e >= m.ne) continue;
     const double mu0 = a.mu0, g0 = a.g0, mb0 = a.mb0;
+    double fb[4][RN];
+#pragma unroll
+    for (int f = 0; f < 4; ++f) load_rows<D>(fb[f], a.fb + f * fs, e, p);
 #pragma unroll
     for (int r = 0; r < RN; ++r) {
       const size_t i = (size_t)e * N + RG * r + p.s;
       if (RG * r + p.s >= N) continue;
-      const double f0 = a.fb[i], f3 = a.fb[3 * fs + i];
-      // fields 6, 7, 8 of the points are at 6, 7, 8
+      const double f0 = fb[0][r], f3 = fb[3][r];
       a.ub[i] = M[0][r] - mb0 * M[7][r];
       a.vb[i] = M[1][r] - mb0 * M[8][r];
       a.hbo[i] = M[6][r] - g0 * (f0 + f3);
       a.qb[i] = M[2][r] + mu0 * f0;
-      a.qb[fs + i] = M[3][r] + mu0 * a.fb[fs + i];
-      a.qb[2 * fs + i] = M[4][r] + mu0 * a.fb[2 * fs + i];
+      a.qb[fs + i] = M[3][r] + mu0 * fb[1][r];
+      a.qb[2 * fs + i] = M[4][r] + mu0 * fb[2][r];
       a.qb[3 * fs + i] = M[5][r] + mu0 * f3;
     }
   }
