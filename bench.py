@@ -512,30 +512,28 @@ def model_counts(cfg, ne, nf):
 
 # DRAM bytes (read + write) per launch of a kernel on a workload, each from one
 # ncu capture of that kernel, with the SHA-256 prefix of the kernel's source
-# file at the capture: a figure is reported only while the source is unchanged
+# files at the capture: a figure is reported only while the source is unchanged
 # (otherwise `traffic` is null, since it would describe another version).
-KERNEL_SOURCE = {"kf_": "spoc_fast.cu", "kx_": "spoc_mixed.cu", "kt_": "spoc_mixed_tc.cu"}
-# At C2 the q-phase and tendency phases are two launches each (the face values
-# once per face, kf_faces, then kf_qphasef / kf_tendf): their figures are the
-# sums over the phase's two kernels.
+KERNEL_SOURCE = {"kf_": ("spoc_tile.cu", "spoc_tile.cuh"),
+                 "kx_": ("spoc_mixed_tile.cu", "spoc_mixed_tile.cuh", "spoc_mixed_dev.cuh")}
+# The q-phase and tendency phases are two launches each (the face values once
+# per face, kt_faces, then kt_qphase / kt_tendency): their figures are the sums
+# over the phase's two kernels.
 NCU_TRAFFIC = {
-    "c2_fs_p6:kf_qphase": (39800320, "3d82445bfb57b56a"),
-    "c2_fs_p6:kf_nlvol": (98205184, "3d82445bfb57b56a"),
-    "c2_fs_p6:kf_tend": (167291904, "3d82445bfb57b56a"),
-    "c3_inv_p7:kx_vol": (248066048, "6bbf3e429a3ee218"),
-    "c3_inv_p7:kx_tend": (578007040, "6bbf3e429a3ee218"),
+    "c2_fs_p6:kf_qphase": (39441920, "cf2fcb640e8af829"),
+    "c2_fs_p6:kf_nlvol": (97395456, "cf2fcb640e8af829"),
+    "c2_fs_p6:kf_tend": (159778304, "cf2fcb640e8af829"),
 }
-# The kernels behind each timed phase of the FP64 nonlinear RHS at the
-# degrees whose modes fit one row per lane (3-6).
-PHASE_KERNELS = {"kf_qphase": "kf_faces<NF=2> (face values of u, v) + kf_qphasef",
-                 "kf_nlvol": "kf_nlvol",
-                 "kf_tend": "kf_faces<NF=6> (face values of f, uh, vh) + kf_tendf"}
+# The kernels behind each timed phase of the FP64 nonlinear RHS.
+PHASE_KERNELS = {"kf_qphase": "kt_faces<NF=2> (face values of u, v) + kt_qphase",
+                 "kf_nlvol": "kt_nlvol",
+                 "kf_tend": "kt_faces<NF=6> (face values of f, uh, vh) + kt_tendency"}
 
 
 def source_digest(kernel: str):
-    for prefix, fname in KERNEL_SOURCE.items():
+    for prefix, names in KERNEL_SOURCE.items():
         if kernel.startswith(prefix):
-            data = (ROOT / "spoc_b200" / "csrc" / fname).read_bytes()
+            data = b"".join((ROOT / "spoc_b200" / "csrc" / f).read_bytes() for f in names)
             return hashlib.sha256(data).hexdigest()[:16]
     return None
 
@@ -1034,7 +1032,7 @@ def main():
             "gpu_launches": int(launches),
             "kernel_ms_per_launch": per_launch_ms,
             "phase_kernels": (PHASE_KERNELS if args.precision == "fp64" and cfg.variant != "lin"
-                              and nm <= 32 else None),
+                              else None),
             "roofline": roof,
             "other_precisions": others,
             "fp64_other_configs": fp64_configs,

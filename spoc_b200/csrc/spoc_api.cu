@@ -72,7 +72,7 @@ struct spoc_handle {
   double *fv = nullptr;  // [nf][6][ngf] face values of the tendency kernel ([nf][4][ngf]: linear)
   double *eterms = nullptr, *escal = nullptr;
   int *flag = nullptr;
-  unsigned *gbar = nullptr;  // grid-barrier word of the multi-step linear kernel
+  unsigned *gbar = nullptr;  // grid-barrier word of the multi-step kernels
   int *lin_order = nullptr;  // element order of its 16-lane tiles (built on first use)
   int lin_norder = 0;
   unsigned long long *cflbits = nullptr;
@@ -851,7 +851,7 @@ int enqueue_steps_fp64(spoc_handle *h, double dt, int nsteps, double *const *bas
   return SPOC_OK;
 }
 
-// FP64 RK4 steps with the state resident: the launches of one step (3 or 1
+// FP64 RK4 steps with the state resident: the launches of one step (1 to 5
 // kernels per stage, the same arguments every step) are captured once as a
 // CUDA graph and replayed, which removes the per-launch host and gap cost
 // that dominates small meshes.  The first step after any change of the
