@@ -417,20 +417,23 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_vol(const MxArgs a, const fl
       ld(T::C_V, m[2]);
       ld(T::C_V + W, m[3]);
       ldw();
+      // the four fields of a point in one store (field by field, a sector of
+      // the record is written four times over: 6.1 -> 7.3 ms per degree-7 step)
+      float *rec = a.trq + (size_t)(valid ? e : 0) * TS * kTrq;
+      for (int c = 0; c < WT; c += 8)
+        if (own(c)) {
+          float v[4][8];
 #pragma unroll
-      for (int f = 0; f < 4; ++f) {
-        float *rec = a.trq + (size_t)(valid ? e : 0) * TS * kTrq + f;
-        for (int c = 0; c < WT; c += 8)
-          if (own(c)) {
-            float v[8];
-            ld(T::S + f * WT + c, v);
-            ldw();
+          for (int f = 0; f < 4; ++f) ld(T::S + f * WT + c, v[f]);
+          ldw();
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-              if (valid && c + j < TG) rec[(c + j) * kTrq] = v[j];
-          }
-        if (valid && half == 0) rec[TG * kTrq] = a.psi0 * m[f][0];
-      }
+          for (int j = 0; j < 8; ++j)
+            if (valid && c + j < TG)
+              *reinterpret_cast<float4 *>(rec + (c + j) * kTrq) = make_float4(v[0][j], v[1][j], v[2][j], v[3][j]);
+        }
+      if (valid && half == 0)
+        *reinterpret_cast<float4 *>(rec + TG * kTrq) =
+            make_float4(a.psi0 * m[0][0], a.psi0 * m[1][0], a.psi0 * m[2][0], a.psi0 * m[3][0]);
     }
 
     // ---- 5. phase B: q at the quadrature points, products, projections
@@ -647,20 +650,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_vol(const MxArgs a, const fl
       ld(T::C_U + W, m0);
       ld(T::C_V, m1);
       ldw();
+      float *rec = a.trq + (size_t)(valid ? e : 0) * TS * kTrq + 4;
+      for (int c = 0; c < WT; c += 8)
+        if (own(c)) {
+          float v[2][8];
+          ld(T::S + 2 * W + c, v[0]);
+          ld(T::S + 2 * W + WT + c, v[1]);
+          ldw();
 #pragma unroll
-      for (int f = 0; f < 2; ++f) {
-        float *rec = a.trq + (size_t)(valid ? e : 0) * TS * kTrq + 4 + f;
-        for (int c = 0; c < WT; c += 8)
-          if (own(c)) {
-            float v[8];
-            ld(T::S + 2 * W + f * WT + c, v);
-            ldw();
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              if (valid && c + j < TG) rec[(c + j) * kTrq] = v[j];
-          }
-        if (valid && half == 0) rec[TG * kTrq] = a.psi0 * (f == 0 ? m0[0] : m1[0]);
-      }
+          for (int j = 0; j < 8; ++j)
+            if (valid && c + j < TG)
+              *reinterpret_cast<float2 *>(rec + (c + j) * kTrq) = make_float2(v[0][j], v[1][j]);
+        }
+      if (valid && half == 0)
+        *reinterpret_cast<float2 *>(rec + TG * kTrq) = make_float2(a.psi0 * m0[0], a.psi0 * m1[0]);
     }
     // the next tile waits on the A buffers before rewriting them; every TMEM
     // read above completed (tcgen05.wait::ld) before the next MMA issue
@@ -834,19 +837,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_tend(const MxArgs a, const f
           if (valid && l < TG) {
             const int side = l / G, j = l - side * G;
             const FaceRef &r = fr[side];
-            const float fqxx = face_value<G, kTrq>(a.trq, r, e, l, j);
-            const float fqxy = face_value<G, kTrq>(a.trq + 1, r, e, l, j);
-            const float fqyx = face_value<G, kTrq>(a.trq + 2, r, e, l, j);
-            const float fqyy = face_value<G, kTrq>(a.trq + 3, r, e, l, j);
-            const float fuh = face_value<G, kTrq>(a.trq + 4, r, e, l, j);
-            const float fvh = face_value<G, kTrq>(a.trq + 5, r, e, l, j);
+            float fq[6];  // qxx, qxy, qyx, qyy, uh, vh
+            face_values<G>(a.trq, r, e, l, j, fq);
             const float fh = face_value<G, kTr>(a.tr_in + 2, r, e, l, j);
-            const float Fxx = a.mu0 * fqxx - a.g0 * fh, Fxy = a.mu0 * fqxy;
-            const float Fyx = a.mu0 * fqyx, Fyy = a.mu0 * fqyy - a.g0 * fh;
+            const float Fxx = a.mu0 * fq[0] - a.g0 * fh, Fxy = a.mu0 * fq[1];
+            const float Fyx = a.mu0 * fq[2], Fyy = a.mu0 * fq[3] - a.g0 * fh;
             const float s = r.sig * di * a.wif[r.sig > 0.f ? j : G - 1 - j];
             x[0][jj] = s * (r.nx * Fxx + r.ny * Fxy);
             x[1][jj] = s * (r.nx * Fyx + r.ny * Fyy);
-            x[2][jj] = -s * (r.nx * fuh + r.ny * fvh);
+            x[2][jj] = -s * (r.nx * fq[4] + r.ny * fq[5]);
           }
         }
 #pragma unroll
@@ -952,8 +951,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_tend(const MxArgs a, const f
         }
         if (a.stage >= 0 && c == 0 && valid) {
           // the mean of each field: the constant mode's coefficient
-#pragma unroll
-          for (int f = 0; f < 3; ++f) a.tr_out[((size_t)e * TS + TG) * kTr + f] = a.psi0 * y[f][0];
+          *reinterpret_cast<float4 *>(a.tr_out + ((size_t)e * TS + TG) * kTr) =
+              make_float4(a.psi0 * y[0][0], a.psi0 * y[1][0], a.psi0 * y[2][0], 0.f);
         }
       }
     if (bad) atomicOr(a.flag, 1);
@@ -968,17 +967,18 @@ __global__ void __launch_bounds__(kTcThreads, 1) kt_tend(const MxArgs a, const f
       p.commit(f);
     }
     p.wait_all();
-#pragma unroll
-    for (int f = 0; f < 3; ++f) {
-      float *rec = a.tr_out + (size_t)(valid ? e : 0) * TS * kTr + f;
+    {
+      float *rec = a.tr_out + (size_t)(valid ? e : 0) * TS * kTr;
       for (int c = 0; c < WT; c += 8)
         if (own(c)) {
-          float v[8];
-          ld(f * WT + c, v);
+          float v[3][8];
+#pragma unroll
+          for (int f = 0; f < 3; ++f) ld(f * WT + c, v[f]);
           ldw();
 #pragma unroll
           for (int jj = 0; jj < 8; ++jj)
-            if (valid && c + jj < TG) rec[(c + jj) * kTr] = v[jj];
+            if (valid && c + jj < TG)
+              *reinterpret_cast<float4 *>(rec + (c + jj) * kTr) = make_float4(v[0][jj], v[1][jj], v[2][jj], 0.f);
         }
     }
     // the trace columns are read before the next tile's lifts overwrite them
