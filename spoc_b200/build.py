@@ -32,7 +32,7 @@ SOURCES = ["spoc_tile.cu", "spoc_kernels.cu", "spoc_fast.cu", "spoc_api.cu", "sp
 VARIANT_SOURCES = [("spoc_fast.cu", "spoc_fast_fma", ["-DSPOC_FMA=1"]),
                    ("spoc_tile.cu", "spoc_tile_fma", ["-DSPOC_FMA=1"])]
 HOST_SOURCES = ["spoc_host.cpp"]
-HEADERS = ["spoc_device.cuh", "spoc_kernels.h", "spoc_launch.h", "spoc_bulk.cuh", "spoc_mixed.h", "spoc_tc.cuh",
+HEADERS = ["spoc_device.cuh", "spoc_kernels.h", "spoc_launch.h", "spoc_barrier.h", "spoc_bulk.cuh", "spoc_mixed.h", "spoc_tc.cuh",
            "spoc_mixed_dev.cuh", "spoc_mixed_tile.cuh", "spoc_tile.cuh"]
 
 

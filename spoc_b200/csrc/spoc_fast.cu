@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "spoc_barrier.h"
 #include "spoc_bulk.cuh"
 #include "spoc_device.cuh"
 #include "spoc_kernels.h"
@@ -1669,7 +1670,7 @@ __global__ void __launch_bounds__(256) kf_lin(DevOps op, DevMesh m, LinArgs a, S
 }
 
 // Grid-wide barrier of a cooperative launch: every block adds one to *count
-// and waits until it reaches `target` (a multiple of the grid size).  The
+// and waits until it reaches `target` (a multiple of the grid size, modulo 2^32).  The
 // wait is bounded: past kGridWaitLimit polls bit 2 of *flag is set and false
 // returned (the caller leaves the kernel).
 constexpr long long kGridWaitLimit = 1ll << 24;
@@ -1685,7 +1686,7 @@ __device__ __forceinline__ bool grid_barrier(unsigned *count, unsigned target, i
     for (long long it = 0; it < kGridWaitLimit; ++it) {
       unsigned v;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-      if (v >= target) {
+      if (barrier_reached(v, target)) {
         done = true;
         break;
       }
