@@ -361,6 +361,10 @@ int check_flag(spoc_handle *h) {
   CK(cudaStreamSynchronize(h->st), "synchronize");
   if (flag) {
     CK(cudaMemsetAsync(h->flag, 0, sizeof(int), h->st), "clear flag");
+    // blocks that gave up left without counting their tiles: the next launch
+    // starts from zero counters again
+    if ((flag & 2) && h->op.sched)
+      CK(cudaMemsetAsync(h->op.sched, 0, sizeof(unsigned) * kTileCounters, h->st), "clear tile counters");
     if (flag & 2) return fail(SPOC_E_CUDA, "wait limit reached in a kernel (tensor-core or bulk-copy barrier)");
     if (flag & 4) return fail(SPOC_E_ARG, "interpol: element id out of range");
     return fail(SPOC_E_NONFINITE, "non-finite tendency detected");

@@ -318,7 +318,8 @@ __device__ __forceinline__ void stage_update(const StageArgs &sa, const StageRow
 // round), the others as the warps come for them: tiles with wall elements
 // cost up to twice the others and come in runs.  sched[0] counts the tiles
 // taken, sched[1] the blocks done; the last block clears both for the next
-// launch.
+// launch.  (A block whose operators did not arrive leaves without done(); the
+// host clears the counters where it reads that error.)
 template <int W>
 struct Tiles {
   unsigned *sched;

@@ -1,0 +1,71 @@
+"""Host side of the library on a stand-in for the CUDA runtime (fake_cudart.cpp):
+what it allocates, captures, launches and clears, and what it does when a call
+fails.  Kernels do nothing there, so no values are looked at."""
+import os
+import subprocess
+import sys
+import textwrap
+from pathlib import Path
+
+import pytest
+
+HERE = Path(__file__).resolve().parent
+CUDA = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
+
+PRELUDE = """
+import ctypes as C
+import sys
+import numpy as np
+from spoc_b200 import api, workloads as W
+fake = C.CDLL(None)
+fake.fake_limit.argtypes = [C.c_size_t]
+fake.fake_held.restype = C.c_size_t
+fake.fake_filled.argtypes, fake.fake_filled.restype = [C.c_size_t], C.c_void_p
+RULES = {3: (12, 4), 4: (25, 5), 5: (27, 6), 6: (33, 7), 7: (42, 9)}
+def problem(nc, variant, n):
+    ng, ngf = RULES[nc]
+    return W.build_problem(W.Config("host", variant, nc, ng, ngf, n, jitter=0.2, beta=2.0e-11, mu0=100.0,
+                                    mb0=1.0e-3, seed=nc, ic="gauss8"))
+def error_of(call, *a):
+    try:
+        call(*a)
+    except api.SpocError as e:
+        return e.code
+    return 0
+"""
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    """Runs a program in a process whose CUDA runtime is the stand-in."""
+    so = tmp_path_factory.mktemp("fake") / "libfake_cudart.so"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I", str(CUDA / "include"),
+                    str(HERE / "fake_cudart.cpp"), "-o", str(so)], check=True)
+
+    def go(program):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + textwrap.dedent(program)], cwd=HERE.parent,
+                           env=dict(os.environ, LD_PRELOAD=str(so)), capture_output=True, text=True, timeout=300)
+        assert r.returncode == 0, r.stdout + r.stderr
+
+    return go
+
+
+@pytest.mark.parametrize("variant", ["fs", "lin"])
+@pytest.mark.parametrize("call", ["cal_var", "rk4_steps"])
+def test_tile_counters_are_cleared_with_a_reported_wait_limit(host, variant, call):
+    """A launch whose operators did not arrive in time leaves the tile counters
+    wherever they were; the call that reports it leaves them zero for the next."""
+    host(f"""
+    p = problem(4, {variant!r}, 45)
+    s = W.make_solver(p)
+    s.set_state(p.u, p.v, p.h)
+    flag = C.c_int.from_address(fake.fake_filled(4))
+    counters = (C.c_uint * 6).from_address(fake.fake_filled(24))
+    call = (lambda: s.rk4_steps(1.0, 1)) if {call!r} == "rk4_steps" else (lambda: s.cal_var(p.u, p.v, p.h))
+    call()
+    flag.value = 2
+    counters[:] = [5, 3, 0, 7, 11, 2]
+    assert error_of(call) == 2
+    assert list(counters) == [0] * 6 and flag.value == 0
+    call()
+    """)
