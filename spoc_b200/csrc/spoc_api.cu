@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -84,7 +85,7 @@ struct spoc_handle {
   // the packed inputs and outputs
   double *bounce_in[3] = {};
   double *bounce[3] = {};
-  double graph_key[6] = {};
+  std::array<double, 6> graph_key{};
   long long graph_launches = 0;
 
   // Allocations of 256 KiB and more come from chunks that grow with the handle
@@ -855,6 +856,15 @@ int enqueue_steps_fp64(spoc_handle *h, double dt, int nsteps, double *const *bas
   return SPOC_OK;
 }
 
+// The scalars in the kernel arguments of a step, and whether the step graph
+// held was captured with them.
+std::array<double, 6> graph_key(const spoc_handle *h, double dt) {
+  return {dt, h->mu0, h->mb0, h->g0, h->hh0, (double)h->path};
+}
+bool graph_is_for(const spoc_handle *h, double dt) {
+  return h->step_graph && h->graph_key == graph_key(h, dt);
+}
+
 // FP64 RK4 steps with the state resident: the launches of one step (1 to 5
 // kernels per stage, the same arguments every step) are captured once as a
 // CUDA graph and replayed, which removes the per-launch host and gap cost
@@ -874,10 +884,7 @@ int graph_steps_fp64(spoc_handle *h, double dt, int nsteps) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   CK(cudaStreamIsCapturing(h->st, &cap), "capture status");
   if (cap != cudaStreamCaptureStatusNone) return enqueue_steps_fp64(h, dt, nsteps);
-  const double key[6] = {dt, h->mu0, h->mb0, h->g0, h->hh0, (double)h->path};
-  bool same = h->step_graph != nullptr;
-  for (int i = 0; i < 6 && same; ++i) same = key[i] == h->graph_key[i];
-  if (!same) {
+  if (!graph_is_for(h, dt)) {
     if (h->step_graph) {
       cudaGraphExecDestroy(h->step_graph);
       h->step_graph = nullptr;
@@ -902,7 +909,7 @@ int graph_steps_fp64(spoc_handle *h, double dt, int nsteps) {
     }
     h->graph_launches = h->launches - l0;
     h->launches = l0;
-    for (int i = 0; i < 6; ++i) h->graph_key[i] = key[i];
+    h->graph_key = graph_key(h, dt);
   }
   for (int it = 0; it < nsteps; ++it) {
     CK(cudaGraphLaunch(h->step_graph, h->st), "graph launch");
@@ -913,15 +920,18 @@ int graph_steps_fp64(spoc_handle *h, double dt, int nsteps) {
 
 // The steps of spoc_rk4_steps_host: the first waits for h's upload, the last
 // stores to the caller's arrays; those between are replayed from the step
-// graph (20 launches a step otherwise, which small and middling meshes wait
-// for: 57 us a step by launches against 37 from the graph at degree 5 on 4050
-// triangles).  Short runs that would have to capture it first go without.
+// graph.  us a step by launches / from the graph: free-slip degree 6 on 8192
+// triangles 577 / 546, on 32768 1684 / 1647; degrees 3 to 5 on 3200 to 9800, where
+// the launches are chained, level within 1 %.  Short runs go without unless the
+// graph held is theirs: they would capture one to replay it a few times.  (Eight
+// steps that do capture one cost within 0.7 % of eight by launches at all of
+// these sizes.)
 int run_steps_host(spoc_handle *h, double dt, int nsteps, double *const *host, int ld,
                    cudaEvent_t sh_ready) {
   constexpr int kGraphFrom = 8;
   const StageArgs probe{};
   const bool one_launch = small_steps(h, probe, 0, nullptr, nullptr) == cudaSuccess;
-  if (one_launch || nsteps < (h->step_graph ? 3 : kGraphFrom))
+  if (one_launch || nsteps < (graph_is_for(h, dt) ? 3 : kGraphFrom))
     return enqueue_steps_fp64(h, dt, nsteps, nullptr, host, ld, sh_ready);
   int rc = enqueue_steps_fp64(h, dt, 1, nullptr, nullptr, 0, sh_ready);
   if (!rc) rc = graph_steps_fp64(h, dt, nsteps - 2);

@@ -69,3 +69,25 @@ def test_tile_counters_are_cleared_with_a_reported_wait_limit(host, variant, cal
     assert list(counters) == [0] * 6 and flag.value == 0
     call()
     """)
+
+
+def test_short_host_runs_keep_the_step_graph_of_another_step_size(host):
+    """Runs on the caller's arrays replay the step graph from eight steps on, and
+    from three where the graph held is theirs; a short run with another step
+    size neither captures one nor drops the one held."""
+    host("""
+    p = problem(4, "fs", 45)
+    s = W.make_solver(p)
+    x = [np.ascontiguousarray(a) for a in (p.u, p.v, p.h)]
+    def graphs(dt, steps):
+        g, l = fake.fake_graphs(), fake.fake_graph_launches()
+        s.rk4_steps_host(*x, dt, steps)
+        return fake.fake_graphs() - g, fake.fake_graph_launches() - l
+    assert graphs(1.0, 7) == (0, 0)
+    assert graphs(1.0, 8) == (1, 5)   # first and last step apart, one before the capture
+    assert graphs(2.0, 4) == (0, 0)
+    assert graphs(2.0, 7) == (0, 0)
+    assert graphs(1.0, 5) == (0, 3)
+    assert graphs(1.0, 3) == (0, 1)
+    assert graphs(1.0, 2) == (0, 0)
+    """)
