@@ -931,7 +931,8 @@ int run_steps_host(spoc_handle *h, double dt, int nsteps, double *const *host, i
   constexpr int kGraphFrom = 8;
   const StageArgs probe{};
   const bool one_launch = small_steps(h, probe, 0, nullptr, nullptr) == cudaSuccess;
-  if (one_launch || nsteps < (graph_is_for(h, dt) ? 3 : kGraphFrom))
+  // (the legacy default stream cannot be captured)
+  if (one_launch || h->st == cudaStreamLegacy || nsteps < (graph_is_for(h, dt) ? 3 : kGraphFrom))
     return enqueue_steps_fp64(h, dt, nsteps, nullptr, host, ld, sh_ready);
   int rc = enqueue_steps_fp64(h, dt, 1, nullptr, nullptr, 0, sh_ready);
   if (!rc) rc = graph_steps_fp64(h, dt, nsteps - 2);

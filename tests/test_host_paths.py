@@ -91,3 +91,18 @@ def test_short_host_runs_keep_the_step_graph_of_another_step_size(host):
     assert graphs(1.0, 3) == (0, 1)
     assert graphs(1.0, 2) == (0, 0)
     """)
+
+
+@pytest.mark.parametrize("variant,n", [("fs", 45), ("lin", 60)])
+def test_host_runs_on_a_stream_that_cannot_be_captured(host, variant, n):
+    """cudaStreamLegacy cannot be captured: runs on the caller's arrays are plain
+    launches there, however long."""
+    host(f"""
+    p = problem(4, {variant!r}, {n})
+    s = W.make_solver(p)
+    s.set_stream(1)
+    x = [np.ascontiguousarray(a) for a in (p.u, p.v, p.h)]
+    for steps in (7, 8, 20):
+        assert error_of(s.rk4_steps_host, *x, 1.0, steps) == 0
+    assert fake.fake_graphs() == 0
+    """)
