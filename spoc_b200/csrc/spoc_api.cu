@@ -12,6 +12,7 @@
 #include <new>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/spoc_gpu.h"
@@ -88,40 +89,50 @@ struct spoc_handle {
   std::array<double, 6> graph_key{};
   long long graph_launches = 0;
 
-  // Allocations of 256 KiB and more come from chunks that grow with the handle
-  // (2 MiB, then as much as is held already, up to 64 MiB at a time): a handle
-  // makes some thirty of them, and each cudaMalloc and cudaFree pair maps and
-  // unmaps memory for 0.1 to 1 ms.  (Smaller ones cost microseconds: the
-  // runtime serves them from its own slabs.)
+  // Buffers made together share one allocation (reserve, then alloc each): a
+  // handle has some thirty, and each cudaMalloc and cudaFree pair maps and unmaps
+  // memory for 0.1 to 1 ms.  No more is asked for than the buffers need, and
+  // where one piece of that size is not to be had they are allocated singly.
   char *chunk = nullptr;
-  size_t chunk_left = 0, held = 0;
+  size_t chunk_left = 0;
+  template <class T>
+  static size_t padded(size_t n) {
+    return (sizeof(T) * (n ? n : 1) + 511) / 512 * 512;
+  }
+  void reserve(size_t bytes) {
+    void *q = nullptr;
+    if (cudaMalloc(&q, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return;
+    }
+    allocs.push_back(q);
+    chunk = static_cast<char *>(q);
+    chunk_left = bytes;
+  }
   template <class T>
   cudaError_t alloc(T **p, size_t n) {
-    const size_t bytes = (sizeof(T) * (n ? n : 1) + 511) / 512 * 512;
-    if (bytes < (256u << 10)) {
+    const size_t bytes = padded<T>(n);
+    if (bytes > chunk_left) {
       const cudaError_t e = cudaMalloc((void **)p, bytes);
       if (e == cudaSuccess) allocs.push_back((void *)*p);
       return e;
-    }
-    if (bytes > chunk_left) {
-      const size_t grow = std::min<size_t>(std::max<size_t>(held, 2u << 20), 64u << 20);
-      const size_t size = std::max(bytes, grow);
-      void *q = nullptr;
-      const cudaError_t e = cudaMalloc(&q, size);
-      if (e != cudaSuccess) return e;
-      allocs.push_back(q);
-      held += size;
-      if (size - bytes >= chunk_left) {  // the fuller of the two chunks is left behind
-        chunk = static_cast<char *>(q) + bytes;
-        chunk_left = size - bytes;
-      }
-      *p = static_cast<T *>(q);
-      return cudaSuccess;
     }
     *p = reinterpret_cast<T *>(chunk);
     chunk += bytes;
     chunk_left -= bytes;
     return cudaSuccess;
+  }
+  // all the buffers that list(take) names by take(pointer, count)
+  template <class L>
+  cudaError_t alloc_all(L &&list) {
+    size_t need = 0;
+    list([&](auto **p, size_t n) { need += padded<std::remove_reference_t<decltype(**p)>>(n); });
+    reserve(need);
+    cudaError_t e = cudaSuccess;
+    list([&](auto **p, size_t n) {
+      if (e == cudaSuccess) e = alloc(p, n);
+    });
+    return e;
   }
   template <class T>
   cudaError_t upload(const T **p, const std::vector<T> &v) {
@@ -283,6 +294,9 @@ int build_mesh(spoc_handle *h, const spoc_mesh *m) {
   DevMesh &d = h->mesh;
   d.ne = ne;
   d.nf = nf;
+  h->reserve(2 * h->padded<int>(itm.size()) + 2 * h->padded<int>(tseg.size()) + h->padded<int>(bdl.size()) +
+             h->padded<double>(norm.size()) + h->padded<double>(vect.size()) +
+             h->padded<double>(normt.size()));
   CK(h->upload(&d.itm, itm), "upload itm");
   CK(h->upload(&d.its, its), "upload its");
   CK(h->upload(&d.tseg, tseg), "upload tseg");
@@ -449,54 +463,59 @@ extern "C" int spoc_create(const spoc_tables *t, const spoc_mesh *m, int variant
   if (!rc) rc = build_mesh(h, m);
   if (!rc) {
     const size_t n = fsize(h);
-    for (int c = 0; c < 3 && ce == cudaSuccess; ++c) {
-      ce = h->alloc(&h->U0[c], n);
-      if (ce == cudaSuccess) ce = h->alloc(&h->SA[c], n);
-      if (ce == cudaSuccess) ce = h->alloc(&h->SB[c], n);
-      if (ce == cudaSuccess) ce = h->alloc(&h->ACC[c], n);
-      if (ce == cudaSuccess) ce = h->alloc(&h->TEND[c], n);
-      if (ce == cudaSuccess) ce = h->alloc(&h->SIN[c], n);
-    }
-    if (ce == cudaSuccess) ce = h->alloc(&h->hb, n);
-    if (ce == cudaSuccess) ce = h->alloc(&h->w0, n);
-    if (ce == cudaSuccess) ce = h->alloc(&h->z0, n);
-    if (ce == cudaSuccess) ce = h->alloc(&h->fc, n);
-    if (variant != SPOC_LIN) {
-      if (ce == cudaSuccess) ce = h->alloc(&h->q, 4 * n);
-      if (ce == cudaSuccess) ce = h->alloc(&h->f, 4 * n);
-      if (ce == cudaSuccess) ce = h->alloc(&h->gx0, n);
-      if (ce == cudaSuccess) ce = h->alloc(&h->gy0, n);
-      if (ce == cudaSuccess) ce = h->alloc(&h->uh, n);
-      if (ce == cudaSuccess) ce = h->alloc(&h->vh, n);
-      if (ce == cudaSuccess) ce = h->alloc(&h->fv, 6 * (size_t)h->ngf * h->nf);
-    }
-    if (ce == cudaSuccess) ce = h->alloc(&h->eterms, 3 * (size_t)h->ne);
-    if (ce == cudaSuccess) ce = h->alloc(&h->escal, 4);
-    if (ce == cudaSuccess) ce = h->alloc(&h->flag, 1);
-    if (ce == cudaSuccess) ce = h->alloc(&h->gbar, 1);
-    if (ce == cudaSuccess) ce = h->alloc(&h->cflbits, 1);
+    const bool fast = fast_available(nc, h->ng, h->ngf);
+    const bool tile = fast && tile_pays(variant, nc, h->ng, h->ngf, h->ne, h->sms);
+    // operator images of the compile-time-sized kernels (bulk-copied into
+    // shared memory by every block)
+    char *img = nullptr, *imgq = nullptr, *imgt = nullptr;
+    ce = h->alloc_all([&](auto &&take) {
+      for (int c = 0; c < 3; ++c) {
+        take(&h->U0[c], n);
+        take(&h->SA[c], n);
+        take(&h->SB[c], n);
+        take(&h->ACC[c], n);
+        take(&h->TEND[c], n);
+        take(&h->SIN[c], n);
+      }
+      take(&h->hb, n);
+      take(&h->w0, n);
+      take(&h->z0, n);
+      take(&h->fc, n);
+      if (variant != SPOC_LIN) {
+        take(&h->q, 4 * n);
+        take(&h->f, 4 * n);
+        take(&h->gx0, n);
+        take(&h->gy0, n);
+        take(&h->uh, n);
+        take(&h->vh, n);
+        take(&h->fv, 6 * (size_t)h->ngf * h->nf);
+      }
+      take(&h->eterms, 3 * (size_t)h->ne);
+      take(&h->escal, 4);
+      take(&h->flag, 1);
+      take(&h->gbar, 1);
+      take(&h->cflbits, 1);
+      if (fast) {
+        take(&img, fast_image_bytes(nc, h->ng, h->ngf, 0));
+        take(&imgq, fast_image_bytes(nc, h->ng, h->ngf, 1));
+      }
+      if (tile) {
+        if (variant == SPOC_LIN) take(&h->fv, 4 * (size_t)h->ngf * h->nf);
+        take(&imgt, tile_image_bytes(nc, h->ng, h->ngf));
+        take(&h->op.sched, kTileCounters);
+      }
+    });
     h->op.flag = h->flag;
-    if (ce == cudaSuccess && fast_available(nc, h->ng, h->ngf)) {
-      // operator images of the compile-time-sized kernels (bulk-copied into
-      // shared memory by every block)
-      void *img = nullptr, *imgq = nullptr;
-      ce = h->alloc(reinterpret_cast<char **>(&img), fast_image_bytes(nc, h->ng, h->ngf, 0));
-      if (ce == cudaSuccess)
-        ce = h->alloc(reinterpret_cast<char **>(&imgq), fast_image_bytes(nc, h->ng, h->ngf, 1));
-      if (ce == cudaSuccess) ce = fast_build_images(h->op, img, imgq, h->st);
+    if (ce == cudaSuccess && fast) {
+      ce = fast_build_images(h->op, img, imgq, h->st);
       h->op.img_ops = img;
       h->op.img_q = imgq;
-      if (ce == cudaSuccess && tile_pays(variant, nc, h->ng, h->ngf, h->ne, h->sms)) {
-        void *imgt = nullptr;
-        if (variant == SPOC_LIN) ce = h->alloc(&h->fv, 4 * (size_t)h->ngf * h->nf);
-        if (ce == cudaSuccess)
-          ce = h->alloc(reinterpret_cast<char **>(&imgt), tile_image_bytes(nc, h->ng, h->ngf));
-        if (ce == cudaSuccess) ce = tile_build_images(h->op, imgt, h->st);
-        if (ce == cudaSuccess) ce = h->alloc(&h->op.sched, kTileCounters);
-        if (ce == cudaSuccess)
-          ce = cudaMemsetAsync(h->op.sched, 0, sizeof(unsigned) * kTileCounters, h->st);
-        h->op.img_tile = imgt;
-      }
+    }
+    if (ce == cudaSuccess && tile) {
+      ce = tile_build_images(h->op, imgt, h->st);
+      if (ce == cudaSuccess)
+        ce = cudaMemsetAsync(h->op.sched, 0, sizeof(unsigned) * kTileCounters, h->st);
+      h->op.img_tile = imgt;
     }
     for (int c = 0; c < 3 && ce == cudaSuccess; ++c)
       ce = cudaMemsetAsync(h->U0[c], 0, sizeof(double) * n, h->st);
@@ -1436,25 +1455,22 @@ int adj_init(spoc_handle *h, AdjCtx *c) {
   if (c->ready) return SPOC_OK;
   const size_t n = fsize(h), ls = (size_t)h->ne * 3 * h->ngf;
   c->n = n;
-  cudaError_t e = cudaSuccess;
-  auto A = [&](double **p, size_t k) {
-    if (e == cudaSuccess) e = h->alloc(p, k);
-  };
-  A(&c->qb, 4 * n); A(&c->qd, 4 * n); A(&c->qs[0], 4 * n); A(&c->qs[1], 4 * n); A(&c->qs[2], 4 * n); A(&c->tgx0, n); A(&c->tgy0, n); A(&c->tuh, n);
-  A(&c->tvh, n); A(&c->tf, 4 * n); A(&c->agx0, n); A(&c->agy0, n); A(&c->auh, n);
-  A(&c->avh, n); A(&c->af, 4 * n); A(&c->aq, 4 * n); A(&c->lx, ls); A(&c->ly, ls);
-  A(&c->lh, ls); A(&c->lq, 4 * ls);
-  for (int i = 0; i < 4; ++i)
-    for (int f = 0; f < 3; ++f) {
-      A(&c->S[i][f], n);
-      A(&c->K[i][f], n);
-    }
-  for (int i = 0; i < 6; ++i)
-    for (int f = 0; f < 3; ++f) A(&c->V[i][f], n);
-  if (h->variant != SPOC_LIN && h->op.img_tile && e == cudaSuccess) {
-    e = h->alloc(&c->img, adj_tile_image_bytes(h->nc, h->ng, h->ngf));
-    if (e == cudaSuccess) e = adj_tile_build_images(h->op, c->img, h->st);
-  }
+  const bool tile = h->variant != SPOC_LIN && h->op.img_tile;
+  cudaError_t e = h->alloc_all([&](auto &&A) {
+    A(&c->qb, 4 * n); A(&c->qd, 4 * n); A(&c->qs[0], 4 * n); A(&c->qs[1], 4 * n); A(&c->qs[2], 4 * n); A(&c->tgx0, n); A(&c->tgy0, n); A(&c->tuh, n);
+    A(&c->tvh, n); A(&c->tf, 4 * n); A(&c->agx0, n); A(&c->agy0, n); A(&c->auh, n);
+    A(&c->avh, n); A(&c->af, 4 * n); A(&c->aq, 4 * n); A(&c->lx, ls); A(&c->ly, ls);
+    A(&c->lh, ls); A(&c->lq, 4 * ls);
+    for (int i = 0; i < 4; ++i)
+      for (int f = 0; f < 3; ++f) {
+        A(&c->S[i][f], n);
+        A(&c->K[i][f], n);
+      }
+    for (int i = 0; i < 6; ++i)
+      for (int f = 0; f < 3; ++f) A(&c->V[i][f], n);
+    if (tile) A(&c->img, adj_tile_image_bytes(h->nc, h->ng, h->ngf));
+  });
+  if (e == cudaSuccess && tile) e = adj_tile_build_images(h->op, c->img, h->st);
   if (e != cudaSuccess) return fail(SPOC_E_NOMEM, "adjoint work space", e);
   c->ready = 1;
   return SPOC_OK;
@@ -1913,6 +1929,7 @@ extern "C" int spoc_bwd_window(spoc_handle *h, int ld, const double *u0, const d
   if (!rc) rc = sweep_params(h, c);
   if (rc) return rc;
   // snapshot buffers
+  if ((int)c->snaps.size() < snaps) h->reserve((snaps - c->snaps.size()) * h->padded<double>(3 * c->n));
   while ((int)c->snaps.size() < snaps) {
     double *p = nullptr;
     cudaError_t e = h->alloc(&p, 3 * c->n);

@@ -10,7 +10,7 @@
 #include <vector>
 
 namespace {
-size_t g_limit = ~(size_t)0, g_held = 0;
+size_t g_limit = ~(size_t)0, g_largest = ~(size_t)0, g_held = 0;
 std::map<void *, size_t> g_mem;
 struct Fill {
   void *at;
@@ -39,6 +39,8 @@ void *token() {
 extern "C" {
 // device memory that may be held at a time
 void fake_limit(size_t bytes) { g_limit = bytes; }
+// and in one piece
+void fake_largest(size_t bytes) { g_largest = bytes; }
 size_t fake_held() { return g_held; }
 // the latest fill of `bytes` bytes
 void *fake_filled(size_t bytes) {
@@ -52,7 +54,7 @@ int fake_launches() { return g_launches; }
 int fake_cooperative() { return g_coop; }
 
 cudaError_t cudaMalloc(void **p, size_t n) {
-  if (n > g_limit || g_held > g_limit - n) return err(cudaErrorMemoryAllocation);
+  if (n > g_largest || n > g_limit || g_held > g_limit - n) return err(cudaErrorMemoryAllocation);
   *p = aligned_alloc(512, (n + 511) / 512 * 512);
   if (!*p) return err(cudaErrorMemoryAllocation);
   memset(*p, 0xff, n);

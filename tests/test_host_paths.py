@@ -18,7 +18,7 @@ import sys
 import numpy as np
 from spoc_b200 import api, workloads as W
 fake = C.CDLL(None)
-fake.fake_limit.argtypes = [C.c_size_t]
+fake.fake_limit.argtypes = fake.fake_largest.argtypes = [C.c_size_t]
 fake.fake_held.restype = C.c_size_t
 fake.fake_filled.argtypes, fake.fake_filled.restype = [C.c_size_t], C.c_void_p
 RULES = {3: (12, 4), 4: (25, 5), 5: (27, 6), 6: (33, 7), 7: (42, 9)}
@@ -26,6 +26,13 @@ def problem(nc, variant, n):
     ng, ngf = RULES[nc]
     return W.build_problem(W.Config("host", variant, nc, ng, ngf, n, jitter=0.2, beta=2.0e-11, mu0=100.0,
                                     mb0=1.0e-3, seed=nc, ic="gauss8"))
+def bytes_needed(p, variant):
+    # the handle's fields and mesh records, without the operators
+    n, ne, nf, g = p.mesh.ne * p.T.nm, p.mesh.ne, p.mesh.nf, p.T.ngf
+    words = 22 * n + 3 * ne + 2 * nf + 7 * ne
+    if variant != "lin":
+        words += 12 * n + 6 * g * nf
+    return 8 * words + 4 * (7 * ne + 4 * nf)
 def error_of(call, *a):
     try:
         call(*a)
@@ -105,4 +112,45 @@ def test_host_runs_on_a_stream_that_cannot_be_captured(host, variant, n):
     for steps in (7, 8, 20):
         assert error_of(s.rk4_steps_host, *x, 1.0, steps) == 0
     assert fake.fake_graphs() == 0
+    """)
+
+
+@pytest.mark.parametrize("nc,variant,n", [(4, "fs", 45), (7, "inv", 30), (5, "fs", 20), (3, "lin", 20)])
+def test_handle_takes_no_more_memory_than_its_buffers(host, nc, variant, n):
+    """A handle fits where its buffers do, in one piece or in pieces of their
+    sizes; what one too large leaves behind does not reach the next."""
+    host(f"""
+    p = problem({nc}, {variant!r}, {n})
+    need, operators = bytes_needed(p, {variant!r}), 2 << 20
+    s = W.make_solver(p)
+    assert need <= fake.fake_held() <= need + operators, (need, fake.fake_held())
+    s.close()
+    assert fake.fake_held() == 0
+    fake.fake_limit(need + operators)
+    s = W.make_solver(p)
+    s.cal_var(p.u, p.v, p.h)
+    s.close()
+    fake.fake_limit(1 << 40)
+    fake.fake_largest(8 * max(4 * p.mesh.ne * p.T.nm, 6 * p.T.ngf * p.mesh.nf) + operators)
+    s = W.make_solver(p)
+    s.cal_var(p.u, p.v, p.h)
+    s.close()
+    fake.fake_limit(need - 4096)
+    assert error_of(W.make_solver, p) == 6
+    assert fake.fake_held() == 0
+    """)
+
+
+def test_gradient_buffers_fit_in_pieces_of_their_sizes(host):
+    host("""
+    p = problem(4, "ns", 45)
+    s = W.make_solver(p)
+    n = p.mesh.ne * p.T.nm
+    before = fake.fake_held()
+    # the largest buffers are the 4 (3 ne) ngf side values
+    fake.fake_largest(8 * 12 * p.mesh.ne * p.T.ngf + 4096)
+    s.set_observations(np.array([1], np.int32), np.ones((1, p.T.nm)), np.array([2], np.int32), np.ones((1, 1)))
+    s.bwd_window((p.u, p.v, p.h), 1.0, 4, 3)
+    work = 8 * (82 * n + 7 * 3 * p.mesh.ne * p.T.ngf)
+    assert fake.fake_held() - before <= work + 3 * 8 * 3 * n + (2 << 20), (fake.fake_held() - before, work)
     """)
