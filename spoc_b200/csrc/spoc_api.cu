@@ -115,6 +115,7 @@ struct spoc_handle {
     if (bytes > chunk_left) {
       const cudaError_t e = cudaMalloc((void **)p, bytes);
       if (e == cudaSuccess) allocs.push_back((void *)*p);
+      else cudaGetLastError();  // not for a later launch to report
       return e;
     }
     *p = reinterpret_cast<T *>(chunk);
@@ -499,11 +500,6 @@ extern "C" int spoc_create(const spoc_tables *t, const spoc_mesh *m, int variant
         take(&img, fast_image_bytes(nc, h->ng, h->ngf, 0));
         take(&imgq, fast_image_bytes(nc, h->ng, h->ngf, 1));
       }
-      if (tile) {
-        if (variant == SPOC_LIN) take(&h->fv, 4 * (size_t)h->ngf * h->nf);
-        take(&imgt, tile_image_bytes(nc, h->ng, h->ngf));
-        take(&h->op.sched, kTileCounters);
-      }
     });
     h->op.flag = h->flag;
     if (ce == cudaSuccess && fast) {
@@ -511,7 +507,14 @@ extern "C" int spoc_create(const spoc_tables *t, const spoc_mesh *m, int variant
       h->op.img_ops = img;
       h->op.img_q = imgq;
     }
-    if (ce == cudaSuccess && tile) {
+    // what the kernels with several elements per warp need beside that: without
+    // it a handle runs one element per warp
+    if (ce == cudaSuccess && tile &&
+        h->alloc_all([&](auto &&take) {
+          if (variant == SPOC_LIN) take(&h->fv, 4 * (size_t)h->ngf * h->nf);
+          take(&imgt, tile_image_bytes(nc, h->ng, h->ngf));
+          take(&h->op.sched, kTileCounters);
+        }) == cudaSuccess) {
       ce = tile_build_images(h->op, imgt, h->st);
       if (ce == cudaSuccess)
         ce = cudaMemsetAsync(h->op.sched, 0, sizeof(unsigned) * kTileCounters, h->st);
@@ -1455,7 +1458,6 @@ int adj_init(spoc_handle *h, AdjCtx *c) {
   if (c->ready) return SPOC_OK;
   const size_t n = fsize(h), ls = (size_t)h->ne * 3 * h->ngf;
   c->n = n;
-  const bool tile = h->variant != SPOC_LIN && h->op.img_tile;
   cudaError_t e = h->alloc_all([&](auto &&A) {
     A(&c->qb, 4 * n); A(&c->qd, 4 * n); A(&c->qs[0], 4 * n); A(&c->qs[1], 4 * n); A(&c->qs[2], 4 * n); A(&c->tgx0, n); A(&c->tgy0, n); A(&c->tuh, n);
     A(&c->tvh, n); A(&c->tf, 4 * n); A(&c->agx0, n); A(&c->agy0, n); A(&c->auh, n);
@@ -1468,9 +1470,11 @@ int adj_init(spoc_handle *h, AdjCtx *c) {
       }
     for (int i = 0; i < 6; ++i)
       for (int f = 0; f < 3; ++f) A(&c->V[i][f], n);
-    if (tile) A(&c->img, adj_tile_image_bytes(h->nc, h->ng, h->ngf));
   });
-  if (e == cudaSuccess && tile) e = adj_tile_build_images(h->op, c->img, h->st);
+  // (without room for the images one element per warp runs)
+  if (e == cudaSuccess && h->variant != SPOC_LIN && h->op.img_tile &&
+      h->alloc(&c->img, adj_tile_image_bytes(h->nc, h->ng, h->ngf)) == cudaSuccess)
+    e = adj_tile_build_images(h->op, c->img, h->st);
   if (e != cudaSuccess) return fail(SPOC_E_NOMEM, "adjoint work space", e);
   c->ready = 1;
   return SPOC_OK;

@@ -154,3 +154,35 @@ def test_gradient_buffers_fit_in_pieces_of_their_sizes(host):
     work = 8 * (82 * n + 7 * 3 * p.mesh.ne * p.T.ngf)
     assert fake.fake_held() - before <= work + 3 * 8 * 3 * n + (2 << 20), (fake.fake_held() - before, work)
     """)
+
+
+@pytest.mark.parametrize("nc,variant,n", [(5, "lin", 50), (7, "fs", 32)])
+def test_kernels_that_need_less_memory_run_where_there_is_none_for_the_others(host, nc, variant, n):
+    """A handle whose fields fit is made, without what the kernels with several
+    elements per warp need beside them; the same for the gradient's buffers."""
+    host(f"""
+    p = problem({nc}, {variant!r}, {n})
+    s = W.make_solver(p)
+    full = fake.fake_held()
+    launches = fake.fake_launches()
+    s.cal_var(p.u, p.v, p.h)
+    tile = fake.fake_launches() - launches
+    s.close()
+    fake.fake_limit(full - 4096)
+    s = W.make_solver(p)
+    launches = fake.fake_launches()
+    s.cal_var(p.u, p.v, p.h)
+    assert (tile, fake.fake_launches() - launches) == ((2, 1) if {variant!r} == "lin" else (5, 3)), (tile, fake.fake_launches() - launches)
+    s.rk4_steps(1.0, 3)
+    s.close()
+    fake.fake_limit(1 << 40)
+    s = W.make_solver(p)
+    before = fake.fake_held()
+    s.adj_rhs((p.u, p.v, p.h), (p.u, p.v, p.h))
+    full = fake.fake_held()
+    s.close()
+    if {variant!r} != "lin":
+        s = W.make_solver(p)
+        fake.fake_limit(full - 4096)
+        s.adj_rhs((p.u, p.v, p.h), (p.u, p.v, p.h))
+    """)
