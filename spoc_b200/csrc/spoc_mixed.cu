@@ -118,9 +118,15 @@ __device__ __forceinline__ void write_traces(const float *o, const float *const 
 #pragma unroll
     for (int f = 0; f < NF; ++f) t[f] = p0 * x[f][0];
   }
-  const size_t off = (size_t)e * TS + lane;
-#pragma unroll
-  for (int f = 0; f < NF; ++f) out[off * FS + f] = t[f];
+  // (a point's record in one store, two for the six-field one)
+  float *rec = out + ((size_t)e * TS + lane) * FS;
+  static_assert((NF == 3 && FS == kTr) || (NF == 6 && FS == kTrq));
+  if constexpr (NF == 3) {
+    *reinterpret_cast<float4 *>(rec) = make_float4(t[0], t[1], t[2], 0.f);
+  } else {
+    *reinterpret_cast<float4 *>(rec) = make_float4(t[0], t[1], t[2], t[3]);
+    *reinterpret_cast<float2 *>(rec + 4) = make_float2(t[4], t[5]);
+  }
 }
 
 // Orthogonal projection of the warp's vector x (shared, length N) onto the
@@ -252,8 +258,9 @@ __device__ __forceinline__ void vol_body(const MxArgs &a, float *sm, int blk, in
     if (lane < TG) {
       const int k = lane / G, j = lane - k * G;
       const FaceRef r = face_ref(a.m, e, k);
-      const float fu = face_value<G, kTr>(a.tr_in, r, e, lane, j);
-      const float fv = face_value<G, kTr>(a.tr_in + 1, r, e, lane, j);
+      float uv[2];
+      face_values<G>(a.tr_in, r, e, lane, j, uv);
+      const float fu = uv[0], fv = uv[1];
       const float s = r.sig * di * o[Dm::WIF + (r.sig > 0.f ? j : G - 1 - j)];
       gl[lane] = s * r.nx * fu;
       gl[TG + lane] = s * r.ny * fu;
@@ -569,19 +576,15 @@ __device__ __forceinline__ void tend_body(const MxArgs &a, float *sm, int blk, i
     if (lane < TG) {
       const int k = lane / G, j = lane - k * G;
       const FaceRef r = face_ref(a.m, e, k);
-      const float fqxx = face_value<G, kTrq>(a.trq, r, e, lane, j);
-      const float fqxy = face_value<G, kTrq>(a.trq + 1, r, e, lane, j);
-      const float fqyx = face_value<G, kTrq>(a.trq + 2, r, e, lane, j);
-      const float fqyy = face_value<G, kTrq>(a.trq + 3, r, e, lane, j);
-      const float fuh = face_value<G, kTrq>(a.trq + 4, r, e, lane, j);
-      const float fvh = face_value<G, kTrq>(a.trq + 5, r, e, lane, j);
+      float fq[6];  // qxx, qxy, qyx, qyy, uh, vh
+      face_values<G>(a.trq, r, e, lane, j, fq);
       const float fh = face_value<G, kTr>(a.tr_in + 2, r, e, lane, j);
-      const float Fxx = a.mu0 * fqxx - a.g0 * fh, Fxy = a.mu0 * fqxy;
-      const float Fyx = a.mu0 * fqyx, Fyy = a.mu0 * fqyy - a.g0 * fh;
+      const float Fxx = a.mu0 * fq[0] - a.g0 * fh, Fxy = a.mu0 * fq[1];
+      const float Fyx = a.mu0 * fq[2], Fyy = a.mu0 * fq[3] - a.g0 * fh;
       const float s = r.sig * di * o[Dm::WIF + (r.sig > 0.f ? j : G - 1 - j)];
       gl[lane] = s * (r.nx * Fxx + r.ny * Fxy);
       gl[TG + lane] = s * (r.nx * Fyx + r.ny * Fyy);
-      gl[2 * TG + lane] = -s * (r.nx * fuh + r.ny * fvh);
+      gl[2 * TG + lane] = -s * (r.nx * fq[4] + r.ny * fq[5]);
     }
     __syncwarp(lane_mask<Dm>());
     float t[3][R];
@@ -674,14 +677,13 @@ __global__ void __launch_bounds__(32 * kMxWarps, Dm::MINB_LIN) kx_lin(const MxAr
     if (lane < TG) {
       const int k = lane / G, j = lane - k * G;
       const FaceRef r = face_ref(a.m, e, k);
-      const float fu = face_value<G, kTr>(a.tr_in, r, e, lane, j);
-      const float fv = face_value<G, kTr>(a.tr_in + 1, r, e, lane, j);
-      const float fh = face_value<G, kTr>(a.tr_in + 2, r, e, lane, j);
+      float f3[3];  // u, v, h
+      face_values<G>(a.tr_in, r, e, lane, j, f3);
       const float s = r.sig * di * o[Dm::WIF + (r.sig > 0.f ? j : G - 1 - j)];
-      const float fxx = -a.g0 * fh;
+      const float fxx = -a.g0 * f3[2];
       gl[lane] = s * r.nx * fxx;
       gl[TG + lane] = s * r.ny * fxx;
-      gl[2 * TG + lane] = -s * a.hh0 * (r.nx * fu + r.ny * fv);
+      gl[2 * TG + lane] = -s * a.hh0 * (r.nx * f3[0] + r.ny * f3[1]);
     }
     __syncwarp(lane_mask<Dm>());
     float t[3][R];

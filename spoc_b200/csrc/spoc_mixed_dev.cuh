@@ -143,24 +143,35 @@ __device__ __forceinline__ float face_value(const float *tr, const FaceRef &r, i
                  (nb[TG * FS] - tr[((size_t)e * TS + TG) * FS]));
 }
 
-// The same for the six fields of a q, uh, vh record array.
-template <int G>
-__device__ __forceinline__ void face_values(const float *trq, const FaceRef &r, int e, int l, int j,
-                                            float (&v)[6]) {
-  constexpr int TG = 3 * G, TS = TG + 1;
-  auto rec = [&](size_t i, float (&x)[6]) {
-    const float4 a = *reinterpret_cast<const float4 *>(trq + i * kTrq);
-    const float2 b = *reinterpret_cast<const float2 *>(trq + i * kTrq + 4);
-    x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w, x[4] = b.x, x[5] = b.y;
+// The same for several fields of a record array, a record at a time: NF = 2 or 3, u, v
+// and h of a stage-input array; 6, qxx, qxy, qyx, qyy, uh, vh.
+template <int G, int NF>
+__device__ __forceinline__ void face_values(const float *tr, const FaceRef &r, int e, int l, int j,
+                                            float (&v)[NF]) {
+  static_assert(NF == 2 || NF == 3 || NF == 6);
+  constexpr int TG = 3 * G, TS = TG + 1, FS = NF == 6 ? kTrq : kTr;
+  auto rec = [&](size_t i, float (&x)[NF]) {
+    const float *p = tr + i * FS;
+    if constexpr (NF == 2) {
+      const float2 a = *reinterpret_cast<const float2 *>(p);
+      x[0] = a.x, x[1] = a.y;
+    } else if constexpr (NF == 3) {
+      const float4 a = *reinterpret_cast<const float4 *>(p);
+      x[0] = a.x, x[1] = a.y, x[2] = a.z;
+    } else {
+      const float4 a = *reinterpret_cast<const float4 *>(p);
+      const float2 b = *reinterpret_cast<const float2 *>(p + 4);
+      x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w, x[4] = b.x, x[5] = b.y;
+    }
   };
   rec((size_t)e * TS + l, v);
   if (r.wall) return;
-  float nb[6], mn[6], mo[6];
+  float nb[NF], mn[NF], mo[NF];
   rec((size_t)r.nb * TS + r.s2 * G + (G - 1 - j), nb);
   rec((size_t)r.nb * TS + TG, mn);
   rec((size_t)e * TS + TG, mo);
 #pragma unroll
-  for (int f = 0; f < 6; ++f) v[f] = 0.5f * (v[f] + nb[f] + (mn[f] - mo[f]));
+  for (int f = 0; f < NF; ++f) v[f] = 0.5f * (v[f] + nb[f] + (mn[f] - mo[f]));
 }
 
 // RK4 bookkeeping of src/shwwnl.f:242-284 on one psi coefficient, FP64, from
