@@ -118,10 +118,13 @@ __device__ __forceinline__ void write_traces(const float *o, const float *const 
 #pragma unroll
     for (int f = 0; f < NF; ++f) t[f] = p0 * x[f][0];
   }
-  // (a point's record in one store, two for the six-field one)
+  // (a point's record in one store; two for the six-field one, three in the
+  // linear variant's)
   float *rec = out + ((size_t)e * TS + lane) * FS;
-  static_assert((NF == 3 && FS == kTr) || (NF == 6 && FS == kTrq));
-  if constexpr (NF == 3) {
+  static_assert((NF == 3 && (FS == kTr || FS == kTrLin)) || (NF == 6 && FS == kTrq));
+  if constexpr (FS == kTrLin) {
+    rec[0] = t[0], rec[1] = t[1], rec[2] = t[2];
+  } else if constexpr (NF == 3) {
     *reinterpret_cast<float4 *>(rec) = make_float4(t[0], t[1], t[2], 0.f);
   } else {
     *reinterpret_cast<float4 *>(rec) = make_float4(t[0], t[1], t[2], t[3]);
@@ -196,7 +199,7 @@ __device__ void wall_vec(const float *o, float *tmp, float (&gx)[Dm::R], float (
 
 // Finishes an element: non-finite check, RK4 update (or tendency output),
 // next stage input and its traces.  t[3][R] holds the psi tendencies.
-template <class Dm>
+template <class Dm, int FS = kTr>
 __device__ void finish_element(const MxArgs &a, const float *o, float *w, int e,
                                float (&t)[3][Dm::R]) {
   constexpr int N = Dm::N;
@@ -225,7 +228,7 @@ __device__ void finish_element(const MxArgs &a, const float *o, float *w, int e,
   if (a.stage < 0) return;
   __syncwarp(lane_mask<Dm>());
   const float *const x[3] = {w, w + N, w + 2 * N};
-  write_traces<Dm, 3, kTr>(o, x, a.tr_out, e);
+  write_traces<Dm, 3, FS>(o, x, a.tr_out, e);
   __syncwarp(lane_mask<Dm>());
 }
 
@@ -721,12 +724,12 @@ __global__ void __launch_bounds__(32 * kMxWarps, Dm::MINB_LIN) kx_lin(const MxAr
       wall_vec<Dm, false>(o, tmp, t[0], t[1], nx, ny);
     }
     __syncwarp(lane_mask<Dm>());
-    finish_element<Dm>(a, o, w, e, t);
+    finish_element<Dm, kTrLin>(a, o, w, e, t);
   }
 }
 
 // Stage input and its traces from the FP64 psi state.
-template <class Dm>
+template <class Dm, int FS>
 __global__ void __launch_bounds__(32 * kMxWarps, Dm::MINB) kx_prep(const MxArgs a) {
   constexpr int N = Dm::N;
   extern __shared__ __align__(16) float sm[];
@@ -747,7 +750,7 @@ __global__ void __launch_bounds__(32 * kMxWarps, Dm::MINB) kx_prep(const MxArgs 
       }
     __syncwarp(lane_mask<Dm>());
     const float *const x[3] = {w, w + N, w + 2 * N};
-    write_traces<Dm, 3, kTr>(o, x, a.tr_out, e);
+    write_traces<Dm, 3, FS>(o, x, a.tr_out, e);
     __syncwarp(lane_mask<Dm>());
   }
 }
@@ -952,6 +955,24 @@ constexpr size_t mx_smem() {
   return sizeof(float) * (Dm::NOPS + (size_t)Dm::SLOTS * Dm::WS);
 }
 
+// Whether the linear kernel is launched behind the one before it in the stream
+// (launch_chained).  us a stage chained / one after the other: degree 4 on 800
+// triangles 5.1 / 7.7, degree 5 on 2048 7.8 / 8.3, on 39200 49.4 / 50.5, degree 6
+// on 8192 16.6 / 18.6, on 131072 202 / 207, degree 7 on 4232 17.1 / 19.6.  Not
+// where the next kernel's blocks crowd a few SMs (degree 6 on 1250 to 2312: 9.1 /
+// 8.3) nor, at degrees 3 and 7, where the state of a run just fits the L2 and the
+// blocks that start early push it out (degree 3 on 61250: 34.8 / 32.8, on 80000:
+// 46.6 / 44; degree 7 on 24200: 80.8 / 75.0; at degrees 4 to 6 the chain still wins
+// there).  (The nonlinear one-element kernels lose by it: degree 6 on 800
+// 19 -> 26.)
+template <class Dm>
+bool lin_chained(int ne, int sms) {
+  if (Dm::N == 28) return ne <= 7 * sms || ne > 16 * sms;
+  // base and accumulator, stage input, two trace arrays
+  const double state = ne * (5.0 * sizeof(float) * 3 * Dm::N + 2.0 * sizeof(float) * kTrLin * Dm::TS);
+  return (Dm::N != 10 && Dm::N != 36) || state < 46e6 || state > 88e6;
+}
+
 // Launches of one right-hand side (stage >= 0: with the RK4 update).
 template <class Dm>
 cudaError_t run_stage(MixedCtx *c, const MxArgs &a, cudaStream_t st, long long *launches,
@@ -965,11 +986,9 @@ cudaError_t run_stage(MixedCtx *c, const MxArgs &a, cudaStream_t st, long long *
     const cudaError_t ge = grid_for(kx_lin<Dm>, smem, c->sms, c->ne, Dm::SLOTS, &g);
     if (ge != cudaSuccess) return ge;
     mark(0);
-    // behind the kernel before it in the stream, unless events are timed between
-    // (degree 4 on 800 elements 7.7 -> 5.4 us; the nonlinear one-element kernels
-    // lose by it, 19 -> 26 us at degree 6 on 800)
+    // (events timed between the kernels want them one after the other)
     cudaError_t le = cudaSuccess;
-    if (!ev) {
+    if (!ev && lin_chained<Dm>(c->ne, c->sms)) {
       le = launch_chained(kx_lin<Dm>, g, 32 * kMxWarps, smem, st, a);
     } else {
       kx_lin<Dm><<<g, 32 * kMxWarps, smem, st>>>(a);
@@ -1021,9 +1040,10 @@ template <class Dm>
 cudaError_t run_prep(MixedCtx *c, const MxArgs &a, cudaStream_t st, long long *launches) {
   constexpr size_t smem = mx_smem<Dm>();
   int g = 0;
-  const cudaError_t ge = grid_for(kx_prep<Dm>, smem, c->sms, c->ne, Dm::SLOTS, &g);
+  const auto kp = c->variant == SPOC_LIN ? kx_prep<Dm, kTrLin> : kx_prep<Dm, kTr>;
+  const cudaError_t ge = grid_for(kp, smem, c->sms, c->ne, Dm::SLOTS, &g);
   if (ge != cudaSuccess) return ge;
-  kx_prep<Dm><<<g, 32 * kMxWarps, smem, st>>>(a);
+  kp<<<g, 32 * kMxWarps, smem, st>>>(a);
   if (launches) *launches += 1;
   return cudaGetLastError();
 }
@@ -1155,8 +1175,8 @@ int mixed_create(MixedCtx **out, const spoc_tables *t, const DevMesh &m, int var
   if (ce == cudaSuccess) ce = c->alloc(&c->k64, 3 * fn);
   if (ce == cudaSuccess) ce = c->alloc(&c->cin, 3 * fn);
   if (ce == cudaSuccess) ce = c->alloc(&c->y, 3 * fn);
-  if (ce == cudaSuccess) ce = c->alloc(&c->tr[0], kTr * tn);
-  if (ce == cudaSuccess) ce = c->alloc(&c->tr[1], kTr * tn);
+  for (float *&tr : c->tr)
+    if (ce == cudaSuccess) ce = c->alloc(&tr, (variant == SPOC_LIN ? kTrLin : kTr) * tn);
   if (ce == cudaSuccess && variant != SPOC_LIN) ce = c->alloc(&c->part, 3 * fn);
   if (ce == cudaSuccess && variant != SPOC_LIN) ce = c->alloc(&c->trq, kTrq * tn);
   if (ce == cudaSuccess) ce = c->alloc(&c->hbq, qn);

@@ -64,9 +64,13 @@ struct __align__(16) SideRef {
   int pad[3];
 };
 
-// Floats per point of the trace records: u, v, h and one unused; q (4), uh,
-// vh, the stage input's h (kernels with several elements per warp) and one unused.
-constexpr int kTr = 4, kTrq = 8;
+// Floats per point of the trace records.  Nonlinear variants: u, v, h and one
+// unused; q (4), uh, vh, the stage input's h (kernels with several elements per
+// warp) and one unused.  Linear variant: u, v, h alone, as the fourth float costs
+// more traffic than one load instead of three saves where a run just fits the L2
+// (degree 3 on 80000 triangles 51 against 47 us a stage; smaller meshes are level
+// within 2 %).
+constexpr int kTr = 4, kTrq = 8, kTrLin = 3;
 
 struct MxArgs {
   int ne;
@@ -74,8 +78,8 @@ struct MxArgs {
   const float *timg;    // operators of the kernels with several elements per warp
   const SideRef *refs;  // [ne][3]
   DevMesh m;
-  const float *tr_in;  // [ne][TS][kTr] trace records of the stage input (u, v, h)
-  float *tr_out;       // [ne][TS][kTr] trace records of the next stage input
+  const float *tr_in;  // [ne][TS][kTr or kTrLin] trace records of the stage input (u, v, h)
+  float *tr_out;       // [ne][TS][kTr or kTrLin] trace records of the next stage input
   float *y;            // [3][ne][N] stage input (FP32); replaced by the next one
   float *part;         // [3][ne][N] partial load vectors (u, v, h)
   float *trq;          // [ne][TS][kTrq] trace records of qxx, qxy, qyx, qyy, uh, vh (h)
@@ -143,21 +147,21 @@ __device__ __forceinline__ float face_value(const float *tr, const FaceRef &r, i
                  (nb[TG * FS] - tr[((size_t)e * TS + TG) * FS]));
 }
 
-// The same for several fields of a record array, a record at a time: NF = 2 or 3, u, v
-// and h of a stage-input array; 6, qxx, qxy, qyx, qyy, uh, vh.
+// The same for several fields of a record array, a record at a time: NF = 2, u
+// and v of a stage-input array; 3, u, v and h of the linear variant's; 6, qxx,
+// qxy, qyx, qyy, uh, vh.
 template <int G, int NF>
 __device__ __forceinline__ void face_values(const float *tr, const FaceRef &r, int e, int l, int j,
                                             float (&v)[NF]) {
   static_assert(NF == 2 || NF == 3 || NF == 6);
-  constexpr int TG = 3 * G, TS = TG + 1, FS = NF == 6 ? kTrq : kTr;
+  constexpr int TG = 3 * G, TS = TG + 1, FS = NF == 6 ? kTrq : (NF == 3 ? kTrLin : kTr);
   auto rec = [&](size_t i, float (&x)[NF]) {
     const float *p = tr + i * FS;
     if constexpr (NF == 2) {
       const float2 a = *reinterpret_cast<const float2 *>(p);
       x[0] = a.x, x[1] = a.y;
     } else if constexpr (NF == 3) {
-      const float4 a = *reinterpret_cast<const float4 *>(p);
-      x[0] = a.x, x[1] = a.y, x[2] = a.z;
+      x[0] = p[0], x[1] = p[1], x[2] = p[2];
     } else {
       const float4 a = *reinterpret_cast<const float4 *>(p);
       const float2 b = *reinterpret_cast<const float2 *>(p + 4);
