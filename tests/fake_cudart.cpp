@@ -7,6 +7,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <string>
 #include <vector>
 
 namespace {
@@ -19,13 +20,16 @@ struct Fill {
 std::vector<Fill> g_fills;
 int g_graphs = 0, g_graph_launches = 0, g_launches = 0, g_coop = 0;
 bool g_capturing = false;
+std::map<const void *, const char *> g_names;
+std::string g_ran;
 cudaError_t g_last = cudaSuccess;
 cudaError_t err(cudaError_t e) {
   if (e != cudaSuccess) g_last = e;
   return e;
 }
-cudaError_t launched() {
+cudaError_t launched(const void *kernel) {
   if (!g_capturing) ++g_launches;
+  g_ran += std::string(g_names.count(kernel) ? g_names[kernel] : "?") + "\n";
   return cudaSuccess;
 }
 // the stream that cannot be captured
@@ -52,6 +56,17 @@ int fake_graphs() { return g_graphs; }
 int fake_graph_launches() { return g_graph_launches; }
 int fake_launches() { return g_launches; }
 int fake_cooperative() { return g_coop; }
+// (mangled) names of the kernels launched since the last call, a line each
+const char *fake_ran() {
+  static std::string r;
+  r.swap(g_ran);
+  g_ran.clear();
+  return r.c_str();
+}
+void __cudaRegisterFunction(void **, const char *host, char *, const char *name, int, uint3 *, uint3 *, dim3 *,
+                            dim3 *, int *) {
+  g_names[host] = name;
+}
 
 cudaError_t cudaMalloc(void **p, size_t n) {
   if (n > g_largest || n > g_limit || g_held > g_limit - n) return err(cudaErrorMemoryAllocation);
@@ -126,11 +141,11 @@ cudaError_t cudaGetLastError(void) {
   g_last = cudaSuccess;
   return e;
 }
-cudaError_t cudaLaunchKernel(const void *, dim3, dim3, void **, size_t, cudaStream_t) { return launched(); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *, const void *, void **) { return launched(); }
-cudaError_t cudaLaunchCooperativeKernel(const void *, dim3, dim3, void **, size_t, cudaStream_t) {
+cudaError_t cudaLaunchKernel(const void *k, dim3, dim3, void **, size_t, cudaStream_t) { return launched(k); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *, const void *k, void **) { return launched(k); }
+cudaError_t cudaLaunchCooperativeKernel(const void *k, dim3, dim3, void **, size_t, cudaStream_t) {
   ++g_coop;
-  return launched();
+  return launched(k);
 }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) {
   *s = (cudaStream_t)token();

@@ -21,6 +21,13 @@ fake = C.CDLL(None)
 fake.fake_limit.argtypes = fake.fake_largest.argtypes = [C.c_size_t]
 fake.fake_held.restype = C.c_size_t
 fake.fake_filled.argtypes, fake.fake_filled.restype = [C.c_size_t], C.c_void_p
+fake.fake_ran.restype = C.c_char_p
+def kernels(call, *a):
+    # names of the kernels a call launches, in order
+    import re
+    fake.fake_ran()
+    call(*a)
+    return re.findall(r"\\d((?:k|kf|kt|kx|ka|k16)_[a-z0-9_]+)", fake.fake_ran().decode())
 RULES = {3: (12, 4), 4: (25, 5), 5: (27, 6), 6: (33, 7), 7: (42, 9)}
 def problem(nc, variant, n):
     ng, ngf = RULES[nc]
@@ -185,4 +192,49 @@ def test_kernels_that_need_less_memory_run_where_there_is_none_for_the_others(ho
         s = W.make_solver(p)
         fake.fake_limit(full - 4096)
         s.adj_rhs((p.u, p.v, p.h), (p.u, p.v, p.h))
+    """)
+
+
+@pytest.mark.parametrize("nc", [3, 4, 5, 6, 7])
+def test_meshes_of_the_gpu_tests_take_the_kernels_they_are_for(host, nc):
+    """On 148 SMs the meshes of test_gpu_tile.py and test_gpu_routes.py run the
+    several-element kernels, the one-launch kernels and the one-element kernels
+    they are sized for."""
+    host(f"""
+    nc = {nc}
+    def state(p):
+        return p.u, p.v, p.h
+    def steps(s, p):
+        s.set_state(*state(p))
+        return s.rk4_steps(1.0, 1)
+    for precision in ("fp64", "fp64_fma"):
+        for variant in ("fs", "ns", "inv"):
+            p = problem(nc, variant, 37)
+            s = W.make_solver(p, precision)
+            right = ["kt_faces", "kt_qphase", "kt_nlvol", "kt_faces", "kt_tendency"]
+            assert kernels(s.cal_var, *state(p)) == right
+            assert kernels(steps, s, p) == 4 * right
+            assert kernels(s.profile_rk4, 1.0, 1) == 4 * right
+        p = problem(nc, "lin", 41)
+        assert kernels(W.make_solver(p, precision).cal_var, *state(p)) == ["kt_faces", "kt_linear"]
+    p = problem(nc, "lin", 61)
+    assert kernels(steps, W.make_solver(p), p) == 4 * ["kt_faces", "kt_linear"]
+    for variant in ("fs", "ns", "inv"):
+        p = problem(nc, variant, 37)
+        s = W.make_solver(p)
+        ran = kernels(s.adj_rhs, state(p), state(p))
+        assert [k for k in ran if k.startswith("ka_")] == ["ka_tend", "ka_faces", "ka_nlvol", "ka_qphase", "ka_faces"]
+        s.set_kernel_path("generic")
+        assert not any(k.startswith(("ka_", "kt_", "kf_")) for k in kernels(s.adj_rhs, state(p), state(p)))
+        p = problem(nc, variant, 41)
+        s = W.make_solver(p, "mixed")
+        mixed = lambda: [k for k in kernels(s.cal_var, *state(p)) if k.startswith(("kx_vol", "kx_tend"))]
+        assert mixed() == ["kx_vol_tile", "kx_tend_tile"]
+        s.set_kernel_path("generic")
+        assert mixed() == ["kx_vol", "kx_tend"]
+        p = problem(nc, variant, 5)
+        s = W.make_solver(p)
+        per_stage = kernels(s.profile_rk4, 1.0, 1)
+        assert len(per_stage) == (20 if nc < 7 else 12) and all(k.startswith("kf_") for k in per_stage), per_stage
+        assert kernels(s.cal_var, *state(p)) == (["kf_nl_steps"] if nc < 7 else per_stage[:3])
     """)
