@@ -35,6 +35,7 @@
 //   kx_lin       calvar_lin.f in one kernel.
 // Face values are the central averages of cal_flu, formed from traces that
 // each element writes for its own three sides (no face arrays).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1294,7 +1295,60 @@ cudaError_t mixed_rhs(MixedCtx *c, const DevMesh &m, const double *const in[3],
 // operators once, runs the volume phase on the member's elements, waits for
 // the whole grid (the face terms of the tendency phase read neighbour trace
 // records), then runs the tendency phase.  All members are free-slip
-// (calvarnl_fs.f); the kernel is in spoc_mixed_tile.cu.
+// (calvarnl_fs.f).  Two kernels: several elements per warp (kx_ens_stage of
+// spoc_mixed_tile.cu), and one, below, for small ensembles.
+namespace {
+
+template <class F>
+__device__ __forceinline__ void ens_dims(int nc, F &&f) {
+  switch (nc) {
+    case 3: f(MDims<3, 12, 4>{}); break;
+    case 4: f(MDims<4, 25, 5>{}); break;
+    case 5: f(MDims<5, 27, 6>{}); break;
+    default: f(MDims<6, 33, 7>{}); break;
+  }
+}
+
+constexpr int kEnsMinBlocks = 4;  // degrees 3-6: one row per lane, 64 registers
+
+// The volume and tendency kernels of each member, a block working on one
+// member.  bt (null except when balancing): each block adds the SM cycles of its
+// volume phase (operator staging included) and of its tendency phase to
+// bt[2 b] and bt[2 b + 1].  (Members and tile counters: kx_ens_stage's.)
+__global__ void __launch_bounds__(32 * kMxWarps, kEnsMinBlocks)
+    kx_ens_small(const EnsMember *__restrict__ mem, const int *__restrict__ blk_member, int, int stage,
+                 int cur, unsigned *, unsigned long long *bt) {
+  extern __shared__ __align__(16) float sm[];
+  const EnsMember &em = mem[blk_member[blockIdx.x]];
+  MxArgs a = em.a;
+  a.stage = stage;
+  a.tr_in = em.tr[cur];
+  a.tr_out = em.tr[cur ^ 1];
+  const int lb = blockIdx.x - em.first_block, nb = em.nblocks;
+  const long long c0 = bt ? clock64() : 0;
+  ens_dims(em.nc, [&](auto d) { stage_mx_ops<decltype(d)>(sm, a.ops); });
+  __syncthreads();
+  ens_dims(em.nc, [&](auto d) { vol_body<decltype(d), SPOC_FS>(a, sm, lb, nb); });
+  if (bt) {
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(bt + 2 * blockIdx.x, (unsigned long long)(clock64() - c0));
+  }
+  cooperative_groups::this_grid().sync();
+  const long long c1 = bt ? clock64() : 0;
+  ens_dims(em.nc, [&](auto d) { tend_body<decltype(d), SPOC_FS>(a, sm, lb, nb); });
+  if (bt) {
+    __syncthreads();
+    if (threadIdx.x == 0) atomicAdd(bt + 2 * blockIdx.x + 1, (unsigned long long)(clock64() - c1));
+  }
+}
+
+EnsKernel ens_small() {
+  const size_t smem = std::max(std::max(mx_smem<MDims<3, 12, 4>>(), mx_smem<MDims<4, 25, 5>>()),
+                               std::max(mx_smem<MDims<5, 27, 6>>(), mx_smem<MDims<6, 33, 7>>()));
+  return {reinterpret_cast<const void *>(kx_ens_small), 32 * kMxWarps, smem};
+}
+
+}  // namespace
 
 struct MixedEns {
   std::vector<MixedCtx *> mem;
@@ -1304,6 +1358,7 @@ struct MixedEns {
   std::vector<int> nb;  // blocks of each member under the current layout
   std::vector<double> mw;  // measured work per member (weight 4)
   int sms = 148, bps = 0, weight = 0, nblk = 0, max_bps = 1;
+  EnsKernel k{};  // of the current layout
   EnsMember *d_mem = nullptr;
   int *d_blk = nullptr;
   unsigned *d_cnt = nullptr;  // tiles taken of each member in a phase
@@ -1322,6 +1377,27 @@ struct MixedEns {
 };
 
 namespace {
+
+// Whether the one-element kernel is the faster under the layout e->nb: where its
+// warps (half-warps at degrees 3 and 4) take one element each and a tile of four
+// would only lengthen their chains.  us a stage here / several elements a warp,
+// four members of one degree: degree 5, 128 elements in all 21 / 25, 4608 (one
+// pass of the 592 blocks) 32 / 37, 6272 (a second pass) 54 / 37; degree 6 21 / 29,
+// 35 / 44, 60 / 44; degree 3 15 / 18 at 128, 20 / 20 at 800, 23 / 22 at 1352; degree 4
+// never (23 / 21, 34 / 28).  Degrees mixed, 3 to 6: 23 / 29 at 128, 29 / 32 at 3200,
+// 46 / 34 at 6272.
+bool ens_small_pays(const MixedEns *e) {
+  int most = 0;
+  long long ne = 0;
+  for (size_t i = 0; i < e->mem.size(); ++i) {
+    const MixedCtx *c = e->mem[i];
+    const int slots = c->nc <= 4 ? MDims<4, 25, 5>::SLOTS : MDims<6, 33, 7>::SLOTS;
+    if (c->ne > (long long)e->nb[i] * slots) return false;
+    most = std::max(most, c->nc);
+    ne += c->ne;
+  }
+  return most >= 5 || (most == 3 && ne <= 8ll * e->sms);
+}
 
 // Blocks per member in proportion to its work, modelled as ne nm^p with
 // p = 2, 1, 0.5, 0 for weight 0..3, or measured (weight 4: the member's
@@ -1365,6 +1441,7 @@ int ens_layout(MixedEns *e) {
     for (int b = 0; b < nb[i]; ++b) blk.push_back(i);
   }
   e->nblk = (int)blk.size();
+  e->k = ens_small_pays(e) ? ens_small() : mixed_tile_ens();
   cudaFree(e->d_mem);
   cudaFree(e->d_blk);
   e->d_mem = nullptr;
@@ -1383,14 +1460,13 @@ int ens_layout(MixedEns *e) {
 }
 
 cudaError_t ens_launch_step(MixedEns *e, int cur0, unsigned long long *bt = nullptr) {
-  const EnsKernel k = mixed_tile_ens();
   int n = (int)e->mem.size();
   for (int s = 0; s < 4; ++s) {
     int stage = s, cur = (cur0 + s) & 1;
     void *args[] = {(void *)&e->d_mem, (void *)&e->d_blk, (void *)&n, (void *)&stage, (void *)&cur,
                     (void *)&e->d_cnt, (void *)&bt};
-    cudaError_t ce = cudaLaunchCooperativeKernel(k.kernel, dim3(e->nblk), dim3(k.threads), args,
-                                                 k.smem, e->st);
+    cudaError_t ce = cudaLaunchCooperativeKernel(e->k.kernel, dim3(e->nblk), dim3(e->k.threads),
+                                                 args, e->k.smem, e->st);
     if (ce != cudaSuccess) return ce;
   }
   return cudaSuccess;
@@ -1420,12 +1496,16 @@ int mixed_ens_create(MixedEns **out, MixedCtx *const *ctx, const DevMesh *meshes
   e->flag.assign(flags, flags + n);
   e->dt.assign(n, 0.0);
   e->sms = sms;
-  const EnsKernel k = mixed_tile_ens();
-  cudaError_t ce = cudaFuncSetAttribute(k.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)k.smem);
-  int occ = 0;
-  if (ce == cudaSuccess)
-    ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.kernel, k.threads, k.smem);
+  // (both kernels have the same blocks resident per SM)
+  cudaError_t ce = cudaSuccess;
+  int occ = 1 << 30;
+  for (const EnsKernel &k : {mixed_tile_ens(), ens_small()}) {
+    int o = 0;
+    if (ce == cudaSuccess)
+      ce = cudaFuncSetAttribute(k.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+    if (ce == cudaSuccess) ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k.kernel, k.threads, k.smem);
+    occ = std::min(occ, o);
+  }
   if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking);
   if (ce == cudaSuccess) ce = cudaMalloc(&e->d_cnt, 2 * sizeof(unsigned) * n);
   if (ce == cudaSuccess) ce = cudaMemset(e->d_cnt, 0, 2 * sizeof(unsigned) * n);

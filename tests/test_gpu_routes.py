@@ -9,6 +9,7 @@ small meshes leave out.
   fused         the FMA form of the several-element kernels
   non-finite    reported by the several-element kernels, the handle usable after
   chained       the linear mixed kernel launched behind the one before it
+  ensemble      both kernels of small ensembles
 """
 import numpy as np
 import pytest
@@ -126,3 +127,26 @@ def test_chained_mixed_linear_steps_match_single_launches(gpu_lib, nc, n):
     ref.profile_rk4(1.0e-3, 3)  # timed between its launches
     for a, b in zip(s.get_state(), ref.get_state()):
         assert np.isfinite(a).all() and np.array_equal(a, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("layout", [(4, 2), (4, 0), (1, 3)])
+@pytest.mark.parametrize("members", [[(5, 4), (6, 5)], [(3, 4), (5, 6), (6, 9)], [(3, 4), (3, 7)], [(4, 4), (3, 4)],
+                                     [(3, 24), (4, 24), (5, 24), (6, 24)], [(6, 30), (3, 5)]])
+def test_small_ensembles_match_members_run_alone(gpu_lib, members, layout):
+    """Either ensemble kernel, a pass of its blocks or several."""
+    ps = [problem(nc, "fs", n) for nc, n in members]
+    alone, mem = [], []
+    for p in ps:
+        for out in (alone, mem):
+            out.append(W.make_solver(p, "mixed"))
+            out[-1].set_state(0.1 * p.u, 0.1 * p.v, 0.1 * p.h)
+    for s in alone:
+        s.rk4_steps(1.0e-3, 5)
+    ens = api.Ensemble(mem)
+    ens.configure(*layout)
+    ens.steps([1.0e-3] * len(ps), 2, graph=False)
+    ens.steps([1.0e-3] * len(ps), 3)
+    for a, b in zip(alone, mem):
+        for x, y in zip(a.get_state(), b.get_state()):
+            assert np.isfinite(x).all() and np.array_equal(x, y)

@@ -238,3 +238,23 @@ def test_meshes_of_the_gpu_tests_take_the_kernels_they_are_for(host, nc):
         assert len(per_stage) == (20 if nc < 7 else 12) and all(k.startswith("kf_") for k in per_stage), per_stage
         assert kernels(s.cal_var, *state(p)) == (["kf_nl_steps"] if nc < 7 else per_stage[:3])
     """)
+
+
+def test_ensemble_kernel_follows_the_members_sizes(host):
+    """Ensembles whose members fit one pass of their blocks take the kernel with
+    one element per warp where that is the faster (148 SMs, one block each here)."""
+    host("""
+    def ens(*members):
+        ps = [problem(nc, "fs", n) for nc, n in members]
+        mem = [W.make_solver(p, "mixed") for p in ps]
+        for p, s in zip(ps, mem):
+            s.set_state(p.u, p.v, p.h)
+        e = api.Ensemble(mem)
+        ran = kernels(lambda: e.steps([1.0] * len(ps), 1, graph=False))
+        return {k for k in ran if k.startswith("kx_ens")}
+    small, tile = {"kx_ens_small"}, {"kx_ens_stage"}
+    assert ens((5, 4), (6, 5)) == ens((3, 4), (5, 6), (6, 9)) == ens((6, 24)) == small
+    assert ens((6, 25)) == ens((3, 12), (6, 25)) == tile
+    assert ens((4, 4), (3, 4)) == ens((4, 20)) == tile
+    assert ens((3, 4), (3, 6)) == ens((3, 24)) == small and ens((3, 25)) == tile
+    """)
