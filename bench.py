@@ -320,8 +320,7 @@ def ensemble_measure(torch, stream, W, api, replicas, rank=0, world=1, count=64,
         "autotuner": {"best": tune["best"], "tried": tune["tried"],
                       "blocks": info["blocks"],
                       "elements_per_block": {"min": float((ne / mb).min()), "max": float((ne / mb).max())},
-                      "warps_per_block": 8,
-                      "elements_per_warp": {"degree 3-4": 2, "degree 5-6": 1}},
+                      "warps_per_block": 4, "elements_per_warp": 4},
         "eta_rel_l2_error_vs_fp64": {"max": float(max(errs)), "median": float(np.median(errs)),
                                      "members": [float(e) for e in errs]},
         "uv_rel_l2_error_vs_fp64": {"max": float(max(uv_errs)),
@@ -520,9 +519,9 @@ KERNEL_SOURCE = {"kf_": ("spoc_tile.cu", "spoc_tile.cuh"),
 # per face, kt_faces, then kt_qphase / kt_tendency): their figures are the sums
 # over the phase's two kernels.
 NCU_TRAFFIC = {
-    "c2_fs_p6:kf_qphase": (39441920, "cf2fcb640e8af829"),
-    "c2_fs_p6:kf_nlvol": (97395456, "cf2fcb640e8af829"),
-    "c2_fs_p6:kf_tend": (159778304, "cf2fcb640e8af829"),
+    "c2_fs_p6:kf_qphase": (39399424, "979ff1f649a58d1f"),
+    "c2_fs_p6:kf_nlvol": (99486208, "979ff1f649a58d1f"),
+    "c2_fs_p6:kf_tend": (159001088, "979ff1f649a58d1f"),
 }
 # The kernels behind each timed phase of the FP64 nonlinear RHS.
 PHASE_KERNELS = {"kf_qphase": "kt_faces<NF=2> (face values of u, v) + kt_qphase",

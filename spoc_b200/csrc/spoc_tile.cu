@@ -16,13 +16,13 @@
 //   * warps are independent (no block barriers after the operator staging)
 //     and own their buffers, filled ahead with cp.async.
 // Measured against one element per warp (spoc_fast.cu) on 32768 triangles, us
-// per right-hand side: degree 3 217 -> 111, 4 358 -> 195, 5 493 -> 281,
-// 6 657 -> 419, 7 1390 -> 693; linear variant 98 -> 38, 132 -> 59, 177 -> 81,
-// 234 -> 119, 623 -> 177.  The FP64 pipe is busy 55 to 63 % of the
-// cycles; ptxas places a product's add right behind it, so a warp alone runs
-// at 44 % of the pipe's rate and three per scheduler (what the registers and
-// the shared memory hold) at about 90 % in the mat-vecs, less in the lifts
-// and the solves.
+// per right-hand side: degree 3 217 -> 105, 4 358 -> 193, 5 493 -> 281,
+// 6 657 -> 413, 7 1390 -> 672; linear variant 98 -> 38, 132 -> 59, 177 -> 81,
+// 234 -> 119, 623 -> 177.  At degree 6 the FP64 pipe is busy 61 to 63 % of the
+// cycles in the element kernels and 34 to 38 % in the face kernels; ptxas
+// places a product's add right behind it, so a warp alone runs at 44 % of the
+// pipe's rate and three per scheduler (what the registers and the shared
+// memory hold) at about 90 % in the mat-vecs, less in the lifts and the solves.
 #include "spoc_tile.cuh"
 
 namespace spoc {
